@@ -90,7 +90,8 @@ struct DevLevel {
   DevBuf<PatchDesc> d_desc;
   DevBuf<int32_t> d_offs, d_runs, d_runs_end;
   DevBuf<float> d_w;
-  DevBuf<int2> d_sw, d_lw, d_run2;
+  DevBuf<int2> d_sw, d_lw;
+  DevBuf<int4> d_run4;
   // Window geometry for a level of width x height: any rotation's raster
   // fits the diagonal; 5x5 placements and centre rounding add 8 cells.
   void set_geometry(size_t width, size_t height) {
@@ -152,10 +153,17 @@ struct DevLevel {
     retire(d_w);
     retire(d_sw);
     retire(d_lw);
-    retire(d_run2);
-    std::vector<int2> run2(runs.size());
-    for (size_t i = 0; i < runs.size(); ++i) run2[i] = make_int2(runs[i], runs_end[i]);
-    d_run2.upload(run2, nullptr);
+    retire(d_run4);
+    std::vector<int4> run4(runs.size());
+    for (const PatchDesc& p : desc) {
+      int32_t before = 0;
+      for (int32_t j = p.run_off; j < p.run_off + p.nruns; ++j) {
+        const int32_t row = runs[size_t(j)] >> 16, begin = int16_t(runs[size_t(j)] & 0xffff), end = runs_end[size_t(j)];
+        run4[size_t(j)] = make_int4(row, begin, end, before);
+        before += end - begin + 1;
+      }
+    }
+    d_run4.upload(run4, nullptr);
     d_desc.upload(desc, nullptr);
     d_sw.upload(sw, nullptr);
     d_lw.upload(lw, nullptr);
@@ -176,7 +184,7 @@ struct DevLevel {
     v.lin_rows = lin_rows;
     v.runs = d_runs.p;
     v.runs_end = d_runs_end.p;
-    v.run2 = d_run2.p;
+    v.run4 = d_run4.p;
     v.npatches = int32_t(desc.size());
     return v;
   }
@@ -1327,6 +1335,16 @@ FindOutput run_find(mvg_ncc_model_s& m, const void* pixels, int type, int64_t W,
       const PatchDesc& d = m.levels[li]->desc[size_t(p)];
       if (!lattice_exact32(d.orow) || !lattice_exact32(d.ocol)) exact32 = false;
     }
+  // staged tracking windows, and the patches off the lattice (never on the tensor cores)
+  int track_window[kMaxLevels] = {};
+  std::vector<std::vector<uint8_t>> off_lattice(level_count);
+  for (size_t li = 0; li < level_count; ++li) {
+    track_window[li] = m.levels[li]->lin_rows;
+    for (int32_t p : plan[li].plist) {
+      const PatchDesc& d = m.levels[li]->desc[size_t(p)];
+      off_lattice[li].push_back(d.orow != 0 || d.ocol != 0);
+    }
+  }
   // longest run of any patch per level (bounds a run's moment sums)
   int max_run[kMaxLevels] = {};
   for (size_t li = 0; li < level_count; ++li)
@@ -1736,6 +1754,19 @@ FindOutput run_find(mvg_ncc_model_s& m, const void* pixels, int type, int64_t W,
       ta.tc_group_of_src = nullptr;
       ta.tc_groups = nullptr;
       ta.dom = dv;
+      ta.win_rows = track_window[t];
+      ta.win_pitch = ((track_window[t] + 3) & ~3) + 4;
+      ta.sel_max = 1;
+      ta.warp_lists = tc[t] != nullptr;
+      for (size_t src = 0; src + 1 < plan[t].sel_off.size(); ++src) {
+        const int32_t b = plan[t].sel_off[src], len = plan[t].sel_off[src + 1] - b;
+        ta.sel_max = std::max(ta.sel_max, std::min(len, 64));
+        int plain = 0;  // patches the tensor cores do not score
+        for (int32_t k = 0; k < len; ++k)
+          plain += !tc[t] || tc[t]->group_of_src[src] < 0 || k >= kTcMaxP ||
+                   off_lattice[t][size_t(plan[t].sel_idx[size_t(b + k)])];
+        if (plain > 2) ta.warp_lists = 0;
+      }
       if (tc[t]) {
         const TcPlan& P = *tc[t];
         const int ng = int(P.groups.size());
@@ -1793,7 +1824,7 @@ FindOutput run_find(mvg_ncc_model_s& m, const void* pixels, int type, int64_t W,
         ta.tc_groups = d_tc_groups[t];
       }
       Span sp(kStTrack, s);
-      check(launch_track(ta, cap, s, ws.smem_optin), "track");
+      check(launch_track(ta, cap, s, ws.smem_optin, ws.sm_count), "track");
     }
     check(cudaMemsetAsync(ws.table.p, 0xff, sizeof(int) * size_t(slots), s), "memset");
     DedupArgs da;

@@ -31,8 +31,6 @@ namespace {
 
 __device__ __forceinline__ int off_row(int32_t o) { return o >> 16; }
 __device__ __forceinline__ int off_col(int32_t o) { return int(int16_t(o & 0xffff)); }
-__device__ __forceinline__ int run_row(int32_t o) { return o >> 16; }
-__device__ __forceinline__ int run_begin(int32_t o) { return int(int16_t(o & 0xffff)); }
 
 __device__ __forceinline__ double dadd(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double dsub(double a, double b) { return __dsub_rn(a, b); }
@@ -131,7 +129,7 @@ __device__ __forceinline__ float window_score(float dot, long long s1, long long
 // prefixes: runs first, first + step, ... (step > 1 splits the runs over
 // threads; the caller adds the parts).
 __device__ __forceinline__ void window_moments(const LevelImage& lev, int pitch, int r, int c,
-                                               const int2* __restrict__ runs, int nruns, long long& s1, long long& s2,
+                                               const int4* __restrict__ runs, int nruns, long long& s1, long long& s2,
                                                int first = 0, int step = 1) {
   s1 = 0;
   s2 = 0;
@@ -140,15 +138,15 @@ __device__ __forceinline__ void window_moments(const LevelImage& lev, int pitch,
     const uint2* __restrict__ P = lev.prefix32;
     int j = first;
     for (; j + 3 * step < nruns; j += 4 * step) {
-      int2 q[4];
+      int4 q[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) q[u] = __ldg(runs + j + u * step);
       uint2 hi[4], lo[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        const size_t base = size_t(r + run_row(q[u].x)) * pitch + c;
-        hi[u] = P[base + q[u].y + 1];
-        lo[u] = P[base + run_begin(q[u].x)];
+        const size_t base = size_t(r + q[u].x) * pitch + c;
+        hi[u] = P[base + q[u].z + 1];
+        lo[u] = P[base + q[u].y];
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
@@ -157,10 +155,10 @@ __device__ __forceinline__ void window_moments(const LevelImage& lev, int pitch,
       }
     }
     for (; j < nruns; j += step) {
-      const int2 q = __ldg(runs + j);
-      const size_t base = size_t(r + run_row(q.x)) * pitch + c;
-      const uint2 hi = P[base + q.y + 1];
-      const uint2 lo = P[base + run_begin(q.x)];
+      const int4 q = __ldg(runs + j);
+      const size_t base = size_t(r + q.x) * pitch + c;
+      const uint2 hi = P[base + q.z + 1];
+      const uint2 lo = P[base + q.y];
       s1 += (long long)(hi.x - lo.x);
       s2 += (long long)(hi.y - lo.y);
     }
@@ -169,18 +167,18 @@ __device__ __forceinline__ void window_moments(const LevelImage& lev, int pitch,
   const longlong2* __restrict__ P = lev.prefix;
   int j = first;
   for (; j + step < nruns; j += 2 * step) {
-    const int2 q0 = __ldg(runs + j), q1 = __ldg(runs + j + step);
-    const size_t b0 = size_t(r + run_row(q0.x)) * pitch + c, b1 = size_t(r + run_row(q1.x)) * pitch + c;
-    const longlong2 h0 = P[b0 + q0.y + 1], l0 = P[b0 + run_begin(q0.x)];
-    const longlong2 h1 = P[b1 + q1.y + 1], l1 = P[b1 + run_begin(q1.x)];
+    const int4 q0 = __ldg(runs + j), q1 = __ldg(runs + j + step);
+    const size_t b0 = size_t(r + q0.x) * pitch + c, b1 = size_t(r + q1.x) * pitch + c;
+    const longlong2 h0 = P[b0 + q0.z + 1], l0 = P[b0 + q0.y];
+    const longlong2 h1 = P[b1 + q1.z + 1], l1 = P[b1 + q1.y];
     s1 += (h0.x - l0.x) + (h1.x - l1.x);
     s2 += (h0.y - l0.y) + (h1.y - l1.y);
   }
   for (; j < nruns; j += step) {
-    const int2 q = __ldg(runs + j);
-    const size_t base = size_t(r + run_row(q.x)) * pitch + c;
-    const longlong2 hi = P[base + q.y + 1];
-    const longlong2 lo = P[base + run_begin(q.x)];
+    const int4 q = __ldg(runs + j);
+    const size_t base = size_t(r + q.x) * pitch + c;
+    const longlong2 hi = P[base + q.z + 1];
+    const longlong2 lo = P[base + q.y];
     s1 += hi.x - lo.x;
     s2 += hi.y - lo.y;
   }
@@ -324,7 +322,7 @@ __global__ void __launch_bounds__(256) coarse_kernel(CoarseArgs a) {
       acc0 = fmaf(__int_as_float(x.y), base[off_row(x.x) * TW + off_col(x.x)] - s0, acc0);
     }
     long long s1, s2;
-    window_moments(a.lev, w + 1, r, c, a.view.run2 + pd.run_off, pd.nruns, s1, s2);
+    window_moments(a.lev, w + 1, r, c, a.view.run4 + pd.run_off, pd.nruns, s1, s2);
     score = window_score(acc0 + acc1, s1, s2, pd.n, a.absolute);
   }
   a.planes[(size_t(p) * h + r) * w + c] = score;
@@ -378,7 +376,7 @@ __global__ void coarse_tc_score_kernel(CoarseTcArgs a) {
     const int ci = (src * a.lat_r + r / 5) * a.lat_c + c / 5;
     const int pos = (r % 5) * 5 + c % 5, k = a.k_of[j];
     long long s1, s2;
-    window_moments(a.lev, w + 1, r, c, a.view.run2 + pd.run_off, pd.nruns, s1, s2);
+    window_moments(a.lev, w + 1, r, c, a.view.run4 + pd.run_off, pd.nruns, s1, s2);
     // sum w (S - S0) = sum w S - S0 sum w (first sample S0)
     const int2 f0 = __ldg(a.view.sw + pd.sample_off);
     const float s0 = a.lev.v[size_t(r + off_row(f0.x)) * w + c + off_col(f0.x)];
@@ -425,285 +423,548 @@ __global__ void nms_kernel(NmsArgs a) {
 }
 
 // ------------------------------------------------------------------ tracking
-// One block per candidate: the target level's query patches inside the
-// candidate's angle window (a precomputed list per source patch), 5x5
-// positions each; the first strict maximum in (patch order, dr, dc) wins
-// (src/ncc_matching/matcher.cpp:670-757).
-//
-// The union image window of all those placements is staged in shared memory,
-// centred on one of its pixels (exact small integers in float) with the
-// level's fixed row pitch, so each sample costs one shared load and one FMA
-// against precomputed linear offsets.  Each thread scores one (patch,
-// position) item, or a slice of its samples when items are few.  Windows
-// larger than the level's staged geometry read the level directly.
-constexpr int kTrackThreads = 256;
+// For every candidate: the target level's query patches inside its angle
+// window (a precomputed list per source patch), 5x5 positions each; the first
+// strict maximum in (patch order, dr, dc) wins (src/ncc_matching/matcher.cpp:
+// 670-757).  Lane p < 25 of a warp holds position (dr, dc) = (p / 5, p mod 5)
+// of one patch at a time.
 constexpr int kTrackMaxSel = 64;
+constexpr int kTrackWarps = 4;          // tensor-core levels: at most this many warps per candidate
+constexpr int kTrackParts = 4;          // column-strip groups of a patch (one warp each)
 
-__global__ void __launch_bounds__(kTrackThreads, 5) track_kernel(TrackArgs a) {
-  extern __shared__ float win[];
-  const int i = blockIdx.x;
-  if (i >= live_count(a.state, a.in_slot)) return;
-  __shared__ int s_sel[kTrackMaxSel];
+// Target patch of a candidate: plist entry, and the centre position on the
+// target level, round((pose - crop - offset) / step - origin).
+struct TrackCentre {
+  float x32r, x32c;
+  double xr, xc;
+};
+__device__ __forceinline__ TrackCentre track_centre(const TrackArgs& a, const Cand& cd) {
+  TrackCentre t{};
+  if (a.exact32) {
+    const float s = float(1.0 / a.step);
+    t.x32r = __fmul_rn(__fsub_rn(__fsub_rn(float(cd.row), float(a.crop_row)), float(a.offset)), s);
+    t.x32c = __fmul_rn(__fsub_rn(__fsub_rn(float(cd.col), float(a.crop_col)), float(a.offset)), s);
+  } else {
+    t.xr = dsub(dsub(cd.row, a.crop_row), a.offset) / a.step;
+    t.xc = dsub(dsub(cd.col, a.crop_col), a.offset) / a.step;
+  }
+  return t;
+}
+__device__ __forceinline__ int track_row(const TrackArgs& a, const TrackCentre& t, double orow) {
+  return a.exact32 ? int(roundf(__fsub_rn(t.x32r, float(orow)))) : int(round(dsub(t.xr, orow)));
+}
+__device__ __forceinline__ int track_col(const TrackArgs& a, const TrackCentre& t, double ocol) {
+  return a.exact32 ? int(roundf(__fsub_rn(t.x32c, float(ocol)))) : int(round(dsub(t.xc, ocol)));
+}
+
+__device__ __forceinline__ bool track_valid(const TrackArgs& a, const PatchDesc& pd, const PosRange& rg, int r, int c) {
+  if (!(r >= rg.r0 && r < rg.r1 && c >= rg.c0 && c < rg.c1)) return false;
+  return !a.dom.mask || may_contain(a.dom, lattice_pose(a.crop_row, a.step, r, pd.orow, a.offset),
+                                    lattice_pose(a.crop_col, a.step, c, pd.ocol, a.offset), a.step);
+}
+
+// Window moments of lane position (dr, dc) at level position (r, c) of one
+// patch; lanes of a warp share the patch.  A lane starts dr runs behind, so
+// that in every step the lanes of all five dr read the same image row (the
+// runs of successive rows begin and end within a few columns of one
+// another): a step's 25 prefix entries lie in one or two cache lines instead
+// of five.  The sums are exact integers, so their order is free.
+__device__ __forceinline__ void lane_moments(const LevelImage& lev, int pitch, int r, int c,
+                                             const int4* __restrict__ runs, int nruns, int dr, long long& s1,
+                                             long long& s2) {
+  s1 = 0;
+  s2 = 0;
+  int at = nruns - dr;
+  while (at < 0) at += nruns;
+  if (at == nruns) at = 0;
+  auto next = [&] {
+    const int4 q = __ldg(runs + at);
+    if (++at == nruns) at = 0;
+    return q;
+  };
+  if (lev.prefix32) {
+    const uint2* __restrict__ P = lev.prefix32;
+    int j = 0;
+    for (; j + 3 < nruns; j += 4) {
+      int4 q[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) q[u] = next();
+      uint2 hi[4], lo[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const size_t base = size_t(r + q[u].x) * pitch + c;
+        hi[u] = P[base + q[u].z + 1];
+        lo[u] = P[base + q[u].y];
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        s1 += (long long)(hi[u].x - lo[u].x);
+        s2 += (long long)(hi[u].y - lo[u].y);
+      }
+    }
+    for (; j < nruns; ++j) {
+      const int4 q = next();
+      const size_t base = size_t(r + q.x) * pitch + c;
+      const uint2 hi = P[base + q.z + 1], lo = P[base + q.y];
+      s1 += (long long)(hi.x - lo.x);
+      s2 += (long long)(hi.y - lo.y);
+    }
+    return;
+  }
+  const longlong2* __restrict__ P = lev.prefix;
+  int j = 0;
+  for (; j + 1 < nruns; j += 2) {
+    const int4 q0 = next(), q1 = next();
+    const size_t b0 = size_t(r + q0.x) * pitch + c, b1 = size_t(r + q1.x) * pitch + c;
+    const longlong2 h0 = P[b0 + q0.z + 1], l0 = P[b0 + q0.y];
+    const longlong2 h1 = P[b1 + q1.z + 1], l1 = P[b1 + q1.y];
+    s1 += (h0.x - l0.x) + (h1.x - l1.x);
+    s2 += (h0.y - l0.y) + (h1.y - l1.y);
+  }
+  if (j < nruns) {
+    const int4 q = next();
+    const size_t base = size_t(r + q.x) * pitch + c;
+    const longlong2 hi = P[base + q.z + 1], lo = P[base + q.y];
+    s1 += hi.x - lo.x;
+    s2 += hi.y - lo.y;
+  }
+}
+
+// Totals of 25 per-lane values over a warp: lane p < 25 returns value p's.
+// Each of the five steps halves the values a lane carries (31 shuffles
+// instead of 125).
+__device__ __forceinline__ float lane_total25(const float (&v)[25]) {
+  const int lane = threadIdx.x & 31;
+  float x[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const float lo = v[i], hi = i + 16 < 25 ? v[i + 16 < 25 ? i + 16 : 0] : 0.f;
+    const bool up = lane & 16;
+    x[i] = (up ? hi : lo) + __shfl_xor_sync(0xffffffffu, up ? lo : hi, 16);
+  }
+#pragma unroll
+  for (int w = 8; w > 0; w >>= 1) {
+    const bool up = lane & w;
+#pragma unroll
+    for (int i = 0; i < w; ++i) {
+      const float lo = x[i], hi = x[i + w];
+      x[i] = (up ? hi : lo) + __shfl_xor_sync(0xffffffffu, up ? lo : hi, w);
+    }
+  }
+  return x[0];
+}
+
+// First and last run of a patch with samples in columns [x0, x1] (a warp's
+// lanes test 32 runs at a time); last < 0 when there is none.
+__device__ __forceinline__ int2 runs_meeting(const int4* __restrict__ runs, int nruns, int x0, int x1) {
+  const int lane = threadIdx.x & 31;
+  int first = INT32_MAX, last = -1;
+  for (int j0 = 0; j0 < nruns; j0 += 32) {
+    bool meets = false;
+    if (j0 + lane < nruns) {
+      const int4 q = __ldg(runs + j0 + lane);
+      meets = q.y <= x1 && q.z >= x0;
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, meets);
+    if (!m) continue;
+    if (first == INT32_MAX) first = j0 + __ffs(m) - 1;
+    last = j0 + 31 - __clz(m);
+  }
+  return make_int2(first, last);
+}
+
+// sum w (S - centre) of one patch at the 25 positions from a window in shared
+// memory (values minus its centre value); lane p < 25 returns position p's.
+// Position (0, 0) puts the patch's row y and column x on window row
+// y + rshift and column x + cshift.  The patch is cut into strips of 16
+// window columns (strip0, strip0 + step, ... are summed): four lanes own four
+// columns each, and the eight groups of four lanes share the runs that meet
+// the strip, so a strip costs about an eighth of its rows.  A lane walks down
+// its rows with the 5 x 8 values under its four samples in registers: per
+// row two 16-byte reads and four weights feed 100 FMAs.
+__device__ __forceinline__ float staged_dots(const float* win, int pitch, const LevelView& view, const PatchDesc& pd,
+                                             int rshift, int cshift, int strip0, int step) {
+  const int lane = threadIdx.x & 31, group = lane >> 2;
+  const int4* __restrict__ runs = view.run4 + pd.run_off;
+  const float* __restrict__ weights = view.w + pd.sample_off;
+  const int xlast = (pd.cmax + cshift) & ~3;  // window columns of the last samples
+  float acc[25];
+#pragma unroll
+  for (int i = 0; i < 25; ++i) acc[i] = 0.f;
+  for (int base = ((pd.cmin + cshift) & ~3) + 16 * strip0; base <= xlast; base += 16 * step) {
+    const int2 span = runs_meeting(runs, pd.nruns, base - cshift, base + 15 - cshift);
+    if (span.y < 0) continue;
+    const int per = (span.y - span.x + 8) >> 3;  // runs per group
+    const int j0 = span.x + group * per, j1 = min(span.y, j0 + per - 1);
+    const int X = min(base + 4 * (lane & 3), xlast);  // past the patch: repeats its last columns, no weights
+    const int x = base + 4 * (lane & 3) - cshift;     // first sample column
+    const float* col = win + X;
+    float v[5][8];  // window row y + i in v[(i + phase) % 5]
+    int ynext = INT32_MIN;
+    for (int it = 0; it < per; it += 5) {
+#pragma unroll
+      for (int phase = 0; phase < 5; ++phase) {
+        const int j = j0 + it + phase;
+        if (it + phase < per && j <= j1) {
+          const int4 q = __ldg(runs + j);
+          const float* row = col + (q.x + rshift) * pitch;
+          if (q.x != ynext) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float4 lo = *reinterpret_cast<const float4*>(row + i * pitch);
+              const float4 hi = *reinterpret_cast<const float4*>(row + i * pitch + 4);
+              float(&r)[8] = v[(phase + i) % 5];
+              r[0] = lo.x, r[1] = lo.y, r[2] = lo.z, r[3] = lo.w, r[4] = hi.x, r[5] = hi.y, r[6] = hi.z, r[7] = hi.w;
+            }
+          }
+          {
+            const float4 lo = *reinterpret_cast<const float4*>(row + 4 * pitch);
+            const float4 hi = *reinterpret_cast<const float4*>(row + 4 * pitch + 4);
+            float(&r)[8] = v[(phase + 4) % 5];
+            r[0] = lo.x, r[1] = lo.y, r[2] = lo.z, r[3] = lo.w, r[4] = hi.x, r[5] = hi.y, r[6] = hi.z, r[7] = hi.w;
+          }
+          ynext = q.x + 1;
+          const unsigned len = unsigned(q.z - q.y);
+          const int u = x - q.y;
+          const float* wp = weights + q.w + u;
+          float w[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) w[e] = unsigned(u + e) <= len ? __ldg(wp + e) : 0.f;
+#pragma unroll
+          for (int i = 0; i < 5; ++i)
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+#pragma unroll
+              for (int d = 0; d < 5; ++d) acc[5 * i + d] = fmaf(w[e], v[(phase + i) % 5][e + d], acc[5 * i + d]);
+        }
+      }
+    }
+  }
+  return lane_total25(acc);
+}
+
+// The same straight from the level, for windows that do not fit shared memory
+// and for single patches: window position (0, 0) is level position (r0, c0);
+// positions outside the level are clamped (they only reach placements that
+// are not scored).  Strips of 32 columns, one per lane.
+struct LevelWindow {
+  const float* v;
+  int w, h, r0, c0;
+  float centre;
+  __device__ __forceinline__ const float* row(int r) const { return v + size_t(min(max(r0 + r, 0), h - 1)) * w; }
+  __device__ __forceinline__ int col(int c) const { return min(max(c0 + c, 0), w - 1); }
+};
+__device__ __forceinline__ float level_dots(const LevelWindow& win, const LevelView& view, const PatchDesc& pd,
+                                            int rshift, int cshift, int strip0, int step) {
+  const int lane = threadIdx.x & 31;
+  const int4* __restrict__ runs = view.run4 + pd.run_off;
+  const float* __restrict__ weights = view.w + pd.sample_off;
+  float acc[25];
+#pragma unroll
+  for (int i = 0; i < 25; ++i) acc[i] = 0.f;
+  for (int x0 = pd.cmin + 32 * strip0; x0 <= pd.cmax; x0 += 32 * step) {
+    const int2 span = runs_meeting(runs, pd.nruns, x0, x0 + 31);
+    const int x = x0 + lane, xc = min(x, pd.cmax) + cshift;
+    for (int j = span.x; j <= span.y; ++j) {
+      const int4 q = __ldg(runs + j);
+      const float w = x >= q.y && x <= q.z ? __ldg(weights + q.w + (x - q.y)) : 0.f;
+#pragma unroll
+      for (int i = 0; i < 5; ++i) {
+        const float* row = win.row(q.x + i + rshift);
+#pragma unroll
+        for (int d = 0; d < 5; ++d) acc[5 * i + d] = fmaf(w, __ldg(row + win.col(xc + d)) - win.centre, acc[5 * i + d]);
+      }
+    }
+  }
+  return lane_total25(acc);
+}
+
+// The tracked candidate from the best item (patch k, position l), or a
+// candidate without a score.
+__device__ void track_write(const TrackArgs& a, int i, const Cand& cd, float best, int item, const TrackCentre& t,
+                            int sel0) {
+  Cand out = cd;
+  out.score = -INFINITY;
+  if (item != INT32_MAX && best > -INFINITY) {
+    const int l = item % 25;
+    const int32_t pi = a.plist[a.sel_idx[sel0 + item / 25]];
+    const PatchDesc pd = a.view.patches[pi];
+    const int r = track_row(a, t, pd.orow) + l / 5 - 2, c = track_col(a, t, pd.ocol) + l % 5 - 2;
+    if (a.exact32) {
+      out.row = double(lattice_pose32(float(a.crop_row), float(a.step), r, float(pd.orow), float(a.offset)));
+      out.col = double(lattice_pose32(float(a.crop_col), float(a.step), c, float(pd.ocol), float(a.offset)));
+    } else {
+      out.row = lattice_pose(a.crop_row, a.step, r, pd.orow, a.offset);
+      out.col = lattice_pose(a.crop_col, a.step, c, pd.ocol, a.offset);
+    }
+    out.angle = pd.angle;
+    out.score = double(best);
+    out.patch = pi;
+  }
+  a.out[i] = out;
+}
+
+// sum w (S - S0) = sum w S - S0 sum w of a patch scored on the tensor cores (first sample S0)
+__device__ __forceinline__ float track_tc_dot(const TrackArgs& a, const PatchDesc& pd, int src, int i, int k, int pos,
+                                              int r, int c) {
+  const int2 f0 = __ldg(a.view.sw + pd.sample_off);
+  const float s0 = a.lev.v[size_t(r + off_row(f0.x)) * a.lev.w + c + off_col(f0.x)];
+  return fmaf(-s0, a.tc_groups[a.tc_group_of_src[src]].weff_k[k],
+              a.tc_dots[size_t(i) * kTcScoreStride + k * 25 + pos]);
+}
+
+// Levels whose lists were scored on the tensor cores, all but at most two
+// patches each (the unrotated patch: its origin is off the lattice): one block
+// of one to four warps per candidate, each warp with its own patches; they add the exact moments,
+// the score and the choice.  The few patches the tensor cores left out are
+// correlated first, by the block.  Bound by the instructions around the
+// prefix loads and their latency.  2048^2 u8, 128^2 template, two steps: 0.27
+// -> 0.17 ms; 57,000 candidates of a 48^2 template over a full circle: 1.03 ->
+// 0.60 ms (one 256-thread block per possible candidate before, each step's
+// lanes on five image rows).
+
+// Dots of patch k of candidate cd, sum w (S - S0), by the whole block, to
+// out[position].  Kept out of line: few candidates need it, and its registers
+// would cost the loop over the moments its occupancy.
+__device__ __noinline__ void plain_dots(const TrackArgs& a, const Cand& cd, int k, float (*part)[32], float* out) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const PatchDesc pd = a.view.patches[a.plist[a.sel_idx[a.sel_off[cd.patch] + k]]];
+  const TrackCentre t = track_centre(a, cd);
+  const int row = track_row(a, t, pd.orow), col = track_col(a, t, pd.ocol);
+  const int cr = min(max(row, 0), a.lev.h - 1), cc = min(max(col, 0), a.lev.w - 1);
+  const LevelWindow win{a.lev.v, a.lev.w, a.lev.h, row - 2, col - 2, a.lev.v[size_t(cr) * a.lev.w + cc]};
+  part[warp][lane] = level_dots(win, a.view, pd, 0, 0, warp, blockDim.x >> 5);
+  __syncthreads();
+  if (warp == 0) {
+    float dot = 0.f;
+    for (int u = 0; u < int(blockDim.x >> 5); ++u) dot += part[u][lane];
+    // sum w (S - S0) = sum w (S - centre) - (S0 - centre) sum w
+    const int2 f0 = __ldg(a.view.sw + pd.sample_off);
+    const float s0 = __ldg(win.row(lane / 5 + off_row(f0.x)) + win.col(lane % 5 + off_col(f0.x)));
+    out[lane] = fmaf(-(s0 - win.centre), pd.wsum, dot);
+    if (lane == 0) atomicAdd(&a.state->track_macs, 25ull * (unsigned long long)pd.n);
+  }
+  __syncthreads();
+}
+
+__global__ void __launch_bounds__(32 * kTrackWarps, 8) track_warp_kernel(const __grid_constant__ TrackArgs a) {
+  __shared__ float s_part[kTrackWarps][32], s_dot[2][32];
+  __shared__ float s_best[kTrackWarps];
+  __shared__ int s_item[kTrackWarps];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const int live = live_count(a.state, a.in_slot);
+  const int dr = lane / 5, dc = lane - 5 * dr;
+  for (int i = blockIdx.x; i < live; i += gridDim.x) {
+    const Cand cd = a.in[i];
+    const int src = cd.patch;
+    const int sel0 = src >= 0 ? a.sel_off[src] : 0;
+    const int n = src >= 0 ? min(a.sel_off[src + 1] - sel0, kTcMaxP) : 0;
+    const bool tc = src >= 0 && a.tc_group_of_src[src] >= 0;
+    // patches without dots
+    bool plain = false;
+    if (lane < n) {
+      const PatchDesc& pd = a.view.patches[a.plist[a.sel_idx[sel0 + lane]]];
+      plain = !tc || pd.orow != 0 || pd.ocol != 0;
+    }
+    const unsigned left = __ballot_sync(0xffffffffu, plain);
+    int slot = 0;
+    for (unsigned todo = left; todo && slot < 2; todo &= todo - 1, ++slot)
+      plain_dots(a, cd, __ffs(todo) - 1, s_part, s_dot[slot]);
+    const TrackCentre t = track_centre(a, cd);
+    float best = -INFINITY;
+    int border = INT32_MAX;
+    for (int k = warp; k < n; k += nwarps) {
+      const int j = a.sel_idx[sel0 + k];
+      const PatchDesc pd = a.view.patches[a.plist[j]];
+      const int r = track_row(a, t, pd.orow) + dr - 2, c = track_col(a, t, pd.ocol) + dc - 2;
+      if (lane >= 25 || !track_valid(a, pd, a.ranges[j], r, c)) continue;
+      const float dot = left >> k & 1 ? s_dot[min(1, __popc(left & ((1u << k) - 1)))][lane]
+                                      : track_tc_dot(a, pd, src, i, k, lane, r, c);
+      long long s1, s2;
+      lane_moments(a.lev, a.lev.w + 1, r, c, a.view.run4 + pd.run_off, pd.nruns, dr, s1, s2);
+      const float sc = window_score(dot, s1, s2, pd.n, a.absolute);
+      if (better(sc, k * 25 + lane, best, border)) {
+        best = sc;
+        border = k * 25 + lane;
+      }
+    }
+    __syncwarp();
+    for (int o = 16; o > 0; o >>= 1) {
+      const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+      const int oo = __shfl_xor_sync(0xffffffffu, border, o);
+      if (better(ob, oo, best, border)) {
+        best = ob;
+        border = oo;
+      }
+    }
+    if (lane == 0) {
+      s_best[warp] = best;
+      s_item[warp] = border;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int w = 1; w < nwarps; ++w)
+        if (better(s_best[w], s_item[w], best, border)) {
+          best = s_best[w];
+          border = s_item[w];
+        }
+      track_write(a, i, cd, best, border, t, sel0);
+    }
+    __syncthreads();
+  }
+}
+
+// Other levels: one block per candidate.  The union window of the patches
+// the block correlates is staged in shared memory, centred on one of its
+// pixels (exact small integers in float; zero outside the level); the warps
+// take (patch, strip group) tasks and (patch, moments) tasks, and then the
+// items are scored.  Windows larger than shared memory read the level.
+// Bound by the instructions of staged_dots (FP32 pipes) and the latency of
+// the small patches' prologues.  uint16 lists, two steps at 2048^2 with a
+// 128^2 template (3.1 G multiply-adds): 1.98 -> 1.09 ms; three at 4096^2 with
+// 256^2 (21 G): 40 -> 5.8 ms (one shared-memory read and one weight read per
+// multiply-add before).
+__global__ void __launch_bounds__(512) track_block_kernel(TrackArgs a) {
+  extern __shared__ float smem[];
   __shared__ int s_row[kTrackMaxSel], s_col[kTrackMaxSel];
   __shared__ unsigned char s_istc[kTrackMaxSel];
-  __shared__ int s_n, s_split, s_wr0, s_wc0, s_wh, s_wcols, s_staged;
-  __shared__ float s_centre;
-  __shared__ float s_part[kTrackThreads];
-  // moment partials of the slices (launches with tensor-core items only)
-  long long* s_m1 = a.split_off >= 0 ? reinterpret_cast<long long*>(win + a.split_off) : nullptr;
-  long long* s_m2 = s_m1 ? s_m1 + kTrackThreads : nullptr;
-  __shared__ float s_wbest[kTrackThreads / 32];
-  __shared__ int s_word[kTrackThreads / 32];
-  const Cand cd = a.in[i];
-  const int WW = a.view.lin_pitch;
-  __shared__ int s_b, s_tc, s_bound[2][4];
-  __shared__ float s_xr32, s_xc32;
-  __shared__ double s_xr, s_xc;
-  if (threadIdx.x == 0) {
+  __shared__ int s_bound[4];
+  __shared__ float s_wbest[16];
+  __shared__ int s_word[16];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+  // dots of the strip groups | moments | window
+  float* s_dot = smem;
+  long long* s_mom = reinterpret_cast<long long*>(smem + size_t(a.sel_max) * kTrackParts * 32);
+  float* win = smem + size_t(a.sel_max) * (kTrackParts * 32 + 2 * 2 * 32);
+  const int live = live_count(a.state, a.in_slot);
+  for (int i = blockIdx.x; i < live; i += gridDim.x) {
+    const Cand cd = a.in[i];
     const int src = cd.patch;
-    const int b = src >= 0 ? a.sel_off[src] : 0, e = src >= 0 ? a.sel_off[src + 1] : 0;
-    s_b = b;
-    s_n = min(e - b, kTrackMaxSel);
-    // rotated patches of a tensor-core group were scored by tc_track_kernel
-    s_tc = a.tc_dots && src >= 0 && a.tc_group_of_src[src] >= 0;
-    // window centres: round((pose - crop - offset) / step - origin)
-    if (a.exact32) {
-      s_xr32 = __fmul_rn(__fsub_rn(__fsub_rn(float(cd.row), float(a.crop_row)), float(a.offset)), float(1.0 / a.step));
-      s_xc32 = __fmul_rn(__fsub_rn(__fsub_rn(float(cd.col), float(a.crop_col)), float(a.offset)), float(1.0 / a.step));
-    } else {
-      s_xr = dsub(dsub(cd.row, a.crop_row), a.offset) / a.step;
-      s_xc = dsub(dsub(cd.col, a.crop_col), a.offset) / a.step;
-    }
-  }
-  __syncthreads();
-  {
-    // one thread per selected patch (at most 64: warps 0 and 1)
-    int wr0 = INT32_MAX, wc0 = INT32_MAX, wr1 = INT32_MIN, wc1 = INT32_MIN;
-    const int k = threadIdx.x;
-    if (k < s_n) {
-      const int j = a.sel_idx[s_b + k];
-      s_sel[k] = j;
-      const PatchDesc pd = a.view.patches[a.plist[j]];
-      int row, col;
-      if (a.exact32) {
-        row = int(roundf(__fsub_rn(s_xr32, float(pd.orow))));
-        col = int(roundf(__fsub_rn(s_xc32, float(pd.ocol))));
-      } else {
-        row = int(round(dsub(s_xr, pd.orow)));
-        col = int(round(dsub(s_xc, pd.ocol)));
-      }
-      s_row[k] = row;
-      s_col[k] = col;
-      const bool istc = s_tc && pd.orow == 0 && pd.ocol == 0 && k < 16;
-      s_istc[k] = istc;
-      const PosRange rg = a.ranges[j];
-      // only placements scored here need image data
-      const int r_lo = max(row - 2, rg.r0), r_hi = min(row + 2, rg.r1 - 1);
-      const int c_lo = max(col - 2, rg.c0), c_hi = min(col + 2, rg.c1 - 1);
-      if (!istc && r_lo <= r_hi && c_lo <= c_hi) {
-        wr0 = r_lo + pd.rmin;
-        wr1 = r_hi + pd.rmax;
-        wc0 = c_lo + pd.cmin;
-        wc1 = c_hi + pd.cmax;
-      }
-    }
-    if (threadIdx.x < 64) {
-      for (int o = 16; o > 0; o >>= 1) {
-        wr0 = min(wr0, __shfl_xor_sync(0xffffffffu, wr0, o));
-        wc0 = min(wc0, __shfl_xor_sync(0xffffffffu, wc0, o));
-        wr1 = max(wr1, __shfl_xor_sync(0xffffffffu, wr1, o));
-        wc1 = max(wc1, __shfl_xor_sync(0xffffffffu, wc1, o));
-      }
-      if ((threadIdx.x & 31) == 0) {
-        s_bound[threadIdx.x >> 5][0] = wr0;
-        s_bound[threadIdx.x >> 5][1] = wr1;
-        s_bound[threadIdx.x >> 5][2] = wc0;
-        s_bound[threadIdx.x >> 5][3] = wc1;
-      }
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const int n = s_n;
-    const int wr0 = min(s_bound[0][0], s_bound[1][0]), wr1 = max(s_bound[0][1], s_bound[1][1]);
-    const int wc0 = min(s_bound[0][2], s_bound[1][2]), wc1 = max(s_bound[0][3], s_bound[1][3]);
-    const int items = n * 25;
-    s_split = items > 0 ? max(1, min(8, kTrackThreads / items)) : 1;
-    const bool any = wr0 <= wr1;
-    s_wr0 = any ? wr0 : 0;
-    s_wc0 = any ? wc0 : 0;
-    s_wh = any ? wr1 - wr0 + 1 : 0;
-    s_wcols = any ? wc1 - wc0 + 1 : 0;
-    s_staged = any && s_wh <= a.view.lin_rows && s_wcols <= WW && a.staged_ok;
-    s_centre = any ? a.lev.v[size_t(wr0 + (wr1 - wr0) / 2) * a.lev.w + wc0 + (wc1 - wc0) / 2] : 0.f;
-  }
-  __syncthreads();
-  const int n = s_n, split = s_split;
-  const int pitch = a.lev.w;
-  const bool staged = s_staged != 0;
-  const int wr0 = s_wr0, wc0 = s_wc0;
-  const float centre = s_centre;
-  if (staged) {
-    const int cols = s_wcols, cells = s_wh * cols;
-    for (int t = threadIdx.x; t < cells; t += kTrackThreads) {
-      const int rr = t / cols, cc = t % cols;
-      win[rr * WW + cc] = a.lev.v[size_t(wr0 + rr) * pitch + wc0 + cc] - centre;
-    }
-  }
-  __syncthreads();
-  float best = -INFINITY;
-  int border = INT32_MAX;
-  const int items = n * 25;
-  const int passes = (items * split + kTrackThreads - 1) / kTrackThreads;
-  for (int pass = 0; pass < passes; ++pass) {
-    // slices are part-major: the lanes of a warp work on neighbouring
-    // placements of one sample (broadcast sample loads)
-    const int t = pass * kTrackThreads + threadIdx.x;
-    const int item = split > 1 ? t % items : t, part = split > 1 ? t / items : 0;
-    bool valid = false, is_tc = false;
-    int r = 0, c = 0;
-    PatchDesc pd{};
-    float acc = 0.f, x0 = 0.f;
-    if (item < items && part < split) {
-      const int k = item / 25, pos = item % 25;
-      const int j = s_sel[k];
-      pd = a.view.patches[a.plist[j]];
-      const PosRange rg = a.ranges[j];
-      r = s_row[k] + pos / 5 - 2;
-      c = s_col[k] + pos % 5 - 2;
-      valid = r >= rg.r0 && r < rg.r1 && c >= rg.c0 && c < rg.c1 &&
-              may_contain(a.dom, lattice_pose(a.crop_row, a.step, r, pd.orow, a.offset),
-                          lattice_pose(a.crop_col, a.step, c, pd.ocol, a.offset), a.step);
-      is_tc = s_istc[k] != 0;
-    }
-    if (is_tc) {
-      // precomputed on the tensor cores
-    } else if (valid && staged) {
-      // sum w (S - centre); the first-sample shift is applied once below
-      const int2* lw = a.view.lw + pd.sample_off;
-      const float* base = win + (r - wr0) * WW + (c - wc0);
-      float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-      int s = part;
-      for (; s + 3 * split < pd.n; s += 4 * split) {
-        const int2 p0 = __ldg(lw + s), p1 = __ldg(lw + s + split), p2 = __ldg(lw + s + 2 * split),
-                   p3 = __ldg(lw + s + 3 * split);
-        a0 = fmaf(__int_as_float(p0.y), base[p0.x], a0);
-        a1 = fmaf(__int_as_float(p1.y), base[p1.x], a1);
-        a2 = fmaf(__int_as_float(p2.y), base[p2.x], a2);
-        a3 = fmaf(__int_as_float(p3.y), base[p3.x], a3);
-      }
-      for (; s < pd.n; s += split) {
-        const int2 p0 = __ldg(lw + s);
-        a0 = fmaf(__int_as_float(p0.y), base[p0.x], a0);
-      }
-      acc = (a0 + a1) + (a2 + a3);
-      if (part == 0) x0 = base[__ldg(lw).x];
-    } else if (valid) {
-      const int2* sw = a.view.sw + pd.sample_off;
-      const float* base = a.lev.v + size_t(r) * pitch + c;
-      const int2 f0 = __ldg(sw);
-      const float s0 = base[off_row(f0.x) * pitch + off_col(f0.x)];
-      float acc1 = 0.f;
-      int s = part;
-      for (; s + split < pd.n; s += 2 * split) {
-        const int2 x = __ldg(sw + s), y = __ldg(sw + s + split);
-        acc = fmaf(__int_as_float(x.y), base[off_row(x.x) * pitch + off_col(x.x)] - s0, acc);
-        acc1 = fmaf(__int_as_float(y.y), base[off_row(y.x) * pitch + off_col(y.x)] - s0, acc1);
-      }
-      if (s < pd.n) {
-        const int2 x = __ldg(sw + s);
-        acc = fmaf(__int_as_float(x.y), base[off_row(x.x) * pitch + off_col(x.x)] - s0, acc);
-      }
-      acc += acc1;
-    }
-    // window moments: with scratch, the runs split over the item's slices
-    // like the samples; otherwise in slice 0
-    long long s1 = 0, s2 = 0;
-    if (valid && (s_m1 || part == 0))
-      window_moments(a.lev, pitch + 1, r, c, a.view.run2 + pd.run_off, pd.nruns, s1,
-                     s2, s_m1 ? part : 0, s_m1 ? split : 1);
-    // combine the slices of one item (threads item + q * items)
-    if (split > 1) {
-      s_part[threadIdx.x] = acc;
-      if (s_m1) {
-        s_m1[threadIdx.x] = s1;
-        s_m2[threadIdx.x] = s2;
-      }
-      __syncthreads();
-    }
-    if (part == 0 && valid) {
-      float dot;
-      if (is_tc) {
-        // sum w (S - S0) = sum w S - S0 sum w (first sample S0)
-        const int k = item / 25;
-        const int2 f0 = __ldg(a.view.sw + pd.sample_off);
-        const float s0 = a.lev.v[size_t(r + off_row(f0.x)) * pitch + c + off_col(f0.x)];
-        dot = fmaf(-s0, a.tc_groups[a.tc_group_of_src[cd.patch]].weff_k[k],
-                   a.tc_dots[size_t(i) * kTcScoreStride + item]);
-      } else {
-        dot = acc;
-        for (int q = 1; q < split; ++q) dot += s_part[threadIdx.x + q * items];
-        // sum w (S - S0) = sum w (S - centre) - (S0 - centre) sum w
-        if (staged) dot = fmaf(-x0, pd.wsum, dot);
-      }
-      if (s_m1)
-        for (int q = 1; q < split; ++q) {
-          s1 += s_m1[threadIdx.x + q * items];
-          s2 += s_m2[threadIdx.x + q * items];
+    const int sel0 = src >= 0 ? a.sel_off[src] : 0;
+    const int n = src >= 0 ? min(a.sel_off[src + 1] - sel0, kTrackMaxSel) : 0;
+    const bool tc = a.tc_dots && src >= 0 && a.tc_group_of_src[src] >= 0;
+    const TrackCentre t = track_centre(a, cd);
+    if (warp == 0) {
+      int wr0 = INT32_MAX, wc0 = INT32_MAX, wr1 = INT32_MIN, wc1 = INT32_MIN;
+      for (int k = lane; k < n; k += 32) {
+        const PatchDesc pd = a.view.patches[a.plist[a.sel_idx[sel0 + k]]];
+        const int row = track_row(a, t, pd.orow), col = track_col(a, t, pd.ocol);
+        s_row[k] = row;
+        s_col[k] = col;
+        const bool istc = tc && pd.orow == 0 && pd.ocol == 0 && k < kTcMaxP;
+        s_istc[k] = istc;
+        if (!istc) {
+          wr0 = min(wr0, row - 2 + pd.rmin);
+          wr1 = max(wr1, row + 2 + pd.rmax);
+          wc0 = min(wc0, col - 2 + pd.cmin);
+          wc1 = max(wc1, col + 2 + pd.cmax);
         }
-      const float sc = window_score(dot, s1, s2, pd.n, a.absolute);
-      if (better(sc, item, best, border)) {
-        best = sc;
-        border = item;
+      }
+      wr0 = __reduce_min_sync(0xffffffffu, wr0);
+      wc0 = __reduce_min_sync(0xffffffffu, wc0);
+      wr1 = __reduce_max_sync(0xffffffffu, wr1);
+      wc1 = __reduce_max_sync(0xffffffffu, wc1);
+      if (lane == 0) {
+        s_bound[0] = wr0;
+        s_bound[1] = wr1;
+        s_bound[2] = wc0;
+        s_bound[3] = wc1;
       }
     }
-    if (split > 1) __syncthreads();
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    const float ob = __shfl_down_sync(0xffffffffu, best, o);
-    const int oo = __shfl_down_sync(0xffffffffu, border, o);
-    if (better(ob, oo, best, border)) {
-      best = ob;
-      border = oo;
+    __syncthreads();
+    const bool any = s_bound[0] <= s_bound[1];  // the block correlates some patch
+    const int wr0 = any ? s_bound[0] : 0, wc0 = any ? s_bound[2] : 0;
+    const int wh = any ? s_bound[1] - wr0 + 1 : 0, ww = any ? s_bound[3] - wc0 + 1 : 0;
+    const bool staged = any && wh <= a.win_rows && ww + 4 <= a.win_pitch;
+    float centre = 0.f;
+    if (any) {
+      const int cr = min(max(wr0 + wh / 2, 0), a.lev.h - 1), cc = min(max(wc0 + ww / 2, 0), a.lev.w - 1);
+      centre = a.lev.v[size_t(cr) * a.lev.w + cc];
     }
-  }
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (lane == 0) {
-    s_wbest[warp] = best;
-    s_word[warp] = border;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float bs = -INFINITY;
-    int bo = INT32_MAX;
-    unsigned long long macs = 0;
-    for (int w = 0; w < kTrackThreads / 32; ++w)
-      if (better(s_wbest[w], s_word[w], bs, bo)) {
-        bs = s_wbest[w];
-        bo = s_word[w];
+    if (staged) {
+      // one warp per row, consecutive columns
+      for (int rr = warp; rr < wh; rr += nwarps) {
+        const int r = wr0 + rr;
+        const bool in = r >= 0 && r < a.lev.h;
+        const float* row = a.lev.v + size_t(in ? r : 0) * a.lev.w + wc0;
+        float* dst = win + rr * a.win_pitch;
+        for (int x = lane; x < min(ww + 4, a.win_pitch); x += 32)
+          dst[x] = in && wc0 + x >= 0 && wc0 + x < a.lev.w ? row[x] - centre : 0.f;
       }
-    for (int k = 0; k < n; ++k)
-      if (!s_istc[k]) macs += 25ull * (unsigned long long)a.view.patches[a.plist[s_sel[k]]].n;
-    atomicAdd(&a.state->track_macs, macs);
-    Cand out = cd;
-    out.score = -INFINITY;
-    if (bo != INT32_MAX && bs > -INFINITY) {
-      const int k = bo / 25, l = bo % 25;
-      const int32_t pi = a.plist[s_sel[k]];
-      const PatchDesc pd = a.view.patches[pi];
-      const int r = s_row[k] + l / 5 - 2, c = s_col[k] + l % 5 - 2;
-      if (a.exact32) {
-        out.row = double(lattice_pose32(float(a.crop_row), float(a.step), r, float(pd.orow), float(a.offset)));
-        out.col = double(lattice_pose32(float(a.crop_col), float(a.step), c, float(pd.ocol), float(a.offset)));
+    }
+    __syncthreads();
+    for (int task = warp; task < n * (kTrackParts + 1); task += nwarps) {
+      const int k = task % n, part = task / n;
+      const int j = a.sel_idx[sel0 + k];
+      const PatchDesc pd = a.view.patches[a.plist[j]];
+      if (part == kTrackParts) {
+        const int dr = lane / 5, dc = lane - 5 * dr;
+        const int r = s_row[k] + dr - 2, c = s_col[k] + dc - 2;
+        long long s1 = 0, s2 = 0;
+        if (lane < 25 && track_valid(a, pd, a.ranges[j], r, c))
+          lane_moments(a.lev, a.lev.w + 1, r, c, a.view.run4 + pd.run_off, pd.nruns, dr, s1, s2);
+        s_mom[k * 32 + lane] = s1;
+        s_mom[(a.sel_max + k) * 32 + lane] = s2;
+      } else if (!s_istc[k]) {
+        const int rs = s_row[k] - 2 - wr0, cs = s_col[k] - 2 - wc0;
+        s_dot[(k * kTrackParts + part) * 32 + lane] =
+            staged ? staged_dots(win, a.win_pitch, a.view, pd, rs, cs, part, kTrackParts)
+                   : level_dots(LevelWindow{a.lev.v, a.lev.w, a.lev.h, wr0, wc0, centre}, a.view, pd, rs, cs, part,
+                                kTrackParts);
+      }
+    }
+    __syncthreads();
+    float best = -INFINITY;
+    int border = INT32_MAX;
+    for (int it = threadIdx.x; it < n * 25; it += blockDim.x) {
+      const int k = it / 25, pos = it - 25 * k;
+      const int j = a.sel_idx[sel0 + k];
+      const PatchDesc pd = a.view.patches[a.plist[j]];
+      const int r = s_row[k] + pos / 5 - 2, c = s_col[k] + pos % 5 - 2;
+      if (!track_valid(a, pd, a.ranges[j], r, c)) continue;
+      float dot;
+      if (s_istc[k]) {
+        dot = track_tc_dot(a, pd, src, i, k, pos, r, c);
       } else {
-        out.row = lattice_pose(a.crop_row, a.step, r, pd.orow, a.offset);
-        out.col = lattice_pose(a.crop_col, a.step, c, pd.ocol, a.offset);
+        dot = 0.f;
+        for (int q = 0; q < kTrackParts; ++q) dot += s_dot[(k * kTrackParts + q) * 32 + pos];
+        // sum w (S - S0) = sum w (S - centre) - (S0 - centre) sum w
+        const int2 f0 = __ldg(a.view.sw + pd.sample_off);
+        const float x0 = a.lev.v[size_t(r + off_row(f0.x)) * a.lev.w + c + off_col(f0.x)] - centre;
+        dot = fmaf(-x0, pd.wsum, dot);
       }
-      out.angle = pd.angle;
-      out.score = double(bs);
-      out.patch = pi;
+      const float sc = window_score(dot, s_mom[k * 32 + pos], s_mom[(a.sel_max + k) * 32 + pos], pd.n, a.absolute);
+      if (better(sc, it, best, border)) {
+        best = sc;
+        border = it;
+      }
     }
-    a.out[i] = out;
+    for (int o = 16; o > 0; o >>= 1) {
+      const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+      const int oo = __shfl_xor_sync(0xffffffffu, border, o);
+      if (better(ob, oo, best, border)) {
+        best = ob;
+        border = oo;
+      }
+    }
+    if (lane == 0) {
+      s_wbest[warp] = best;
+      s_word[warp] = border;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      unsigned long long macs = 0;
+      for (int w = 0; w < nwarps; ++w)
+        if (better(s_wbest[w], s_word[w], best, border)) {
+          best = s_wbest[w];
+          border = s_word[w];
+        }
+      for (int k = 0; k < n; ++k)
+        if (!s_istc[k]) macs += 25ull * (unsigned long long)a.view.patches[a.plist[a.sel_idx[sel0 + k]]].n;
+      if (macs) atomicAdd(&a.state->track_macs, macs);
+      track_write(a, i, cd, best, border, t, sel0);
+    }
+    __syncthreads();
   }
 }
 
@@ -2302,28 +2563,32 @@ cudaError_t launch_nms(const NmsArgs& a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_track(const TrackArgs& a, int max_candidates, cudaStream_t s, size_t smem_limit) {
+cudaError_t launch_track(const TrackArgs& a, int max_candidates, cudaStream_t s, size_t smem_limit, int sms) {
+  // candidates are strided over a grid that fills the GPU a few times: the
+  // list's length is only known on the device, and a block per possible
+  // candidate costs more than the work when the budget is large (65536
+  // blocks: about 60 us)
+  if (a.warp_lists) {
+    // a warp for every four patches of the longest list: a 128^2 template's
+    // lists of nine take 0.17 ms with four warps and 0.22 ms with one, a 48^2
+    // template's lists of three 0.78 and 0.60 ms (57,000 candidates)
+    const int warps = a.sel_max <= 4 ? 1 : a.sel_max <= 8 ? 2 : kTrackWarps;
+    track_warp_kernel<<<std::min(max_candidates, 96 / warps * sms), 32 * warps, 0, s>>>(a);
+    return cudaGetLastError();
+  }
   TrackArgs b = a;
-  size_t smem = size_t(a.view.lin_pitch) * size_t(a.view.lin_rows) * sizeof(float);
-  const size_t fixed = 8 * 1024;  // static shared memory of the kernel
-  const size_t scratch = a.tc_dots ? 2 * kTrackThreads * sizeof(long long) : 0;
-  if (smem + scratch + fixed > smem_limit || smem > 160 * 1024) {
-    b.staged_ok = 0;
+  const size_t tables = size_t(a.sel_max) * (kTrackParts * 32 + 2 * 2 * 32) * sizeof(float);
+  const size_t fixed = 4 * 1024;  // static and reserved shared memory of the kernel
+  size_t smem = size_t(a.win_pitch) * size_t(a.win_rows) * sizeof(float);
+  if (smem + tables + fixed > smem_limit) {
+    b.win_rows = b.win_pitch = 0;
     smem = 0;
-  } else {
-    b.staged_ok = 1;
   }
-  // tensor-core items leave the sample slices idle: they split the runs
-  // instead, through a scratch after the window
-  if (scratch) {
-    smem = (smem + 15) & ~size_t(15);  // 8-byte entries: start on a 16-byte boundary
-    b.split_off = int(smem / sizeof(float));
-    smem += scratch;
-  } else {
-    b.split_off = -1;
-  }
-  if (const cudaError_t e = reserve_dynamic_smem(reinterpret_cast<const void*>(track_kernel), smem)) return e;
-  track_kernel<<<max_candidates, kTrackThreads, smem, s>>>(b);
+  smem += tables;
+  if (const cudaError_t e = reserve_dynamic_smem(reinterpret_cast<const void*>(track_block_kernel), smem)) return e;
+  // a window that leaves room for one block per SM gets 16 warps, others 8
+  const int threads = smem > 100 * 1024 ? 512 : 256;
+  track_block_kernel<<<std::min(max_candidates, 16 * sms), threads, smem, s>>>(b);
   return cudaGetLastError();
 }
 

@@ -116,12 +116,13 @@ struct TrackArgs {
   double crop_row, crop_col, step, offset;
   int exact32;              // lattice arithmetic is exact in FP32 (host-checked)
   int absolute;
-  int staged_ok;            // set by the launcher: dynamic shared memory holds the window
-  int split_off;            // set by the launcher: float offset of the moment-split scratch in
-                            // dynamic shared memory (-1: no scratch, moments in one slice)
+  int sel_max;              // longest list of selected patches (at most 64)
+  int win_rows, win_pitch;  // staged window: rows, floats per row (0: set by the launcher when it does not fit)
+  int warp_lists;           // 1: the tensor cores scored all but at most two patches of every list
   // sum w S of the rotated patches of tensor-core groups (nullable),
-  // kTcScoreStride per candidate, and their groups (for weff_k)
-  const float* tc_dots;
+  // kTcScoreStride per candidate, and their groups (for weff_k); the other
+  // patches' dots join them where warp_lists is set
+  float* tc_dots;
   const int32_t* tc_group_of_src;
   const TcGroup* tc_groups;
   DomainView dom;
@@ -374,7 +375,7 @@ cudaError_t launch_pyramid(const LevelImage& src, LevelImage dst, int32_t* error
 cudaError_t launch_prefix(const LevelImage& lev, cudaStream_t s);
 cudaError_t launch_coarse(const CoarseArgs& a, int max_bh, int max_bw, cudaStream_t s, size_t smem_limit);
 cudaError_t launch_nms(const NmsArgs& a, cudaStream_t s);
-cudaError_t launch_track(const TrackArgs& a, int max_candidates, cudaStream_t s, size_t smem_limit);
+cudaError_t launch_track(const TrackArgs& a, int max_candidates, cudaStream_t s, size_t smem_limit, int sms);
 cudaError_t launch_dedup(const DedupArgs& a, int max_candidates, cudaStream_t s);
 cudaError_t launch_score(const ScoreArgs& a, int max_candidates, cudaStream_t s);
 cudaError_t launch_adjoint(const AdjointArgs& a, cudaStream_t s);
