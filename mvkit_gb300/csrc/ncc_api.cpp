@@ -681,7 +681,7 @@ struct Workspace {
   DevBuf<longlong2> lev_p[kMaxLevels];
   DevBuf<float> planes;
   DevBuf<Cand> cand_a, cand_b, tmp, sorted, accepted;
-  DevBuf<unsigned long long> sort_keys;  // bitonic sort of long lists (budgets above kRankSortMax)
+  DevBuf<unsigned long long> sort_keys;  // candidate sort: two (key, index) lists
   DevBuf<int32_t> sort_idx;
   DevBuf<RectAux> aux, accepted_aux;
   DevBuf<int32_t> tested;
@@ -1855,6 +1855,12 @@ FindOutput run_find(mvg_ncc_model_s& m, const void* pixels, int type, int64_t W,
   }
 
   // full-resolution score (matcher.cpp:813-822) and sort (824-827)
+  RectGeom geom;
+  geom.left = -base.ocol - .5;
+  geom.right = double(base.width) - base.ocol - .5;
+  geom.top = -base.orow - .5;
+  geom.bottom = double(base.height) - base.orow - .5;
+  geom.area = double(base.width) * double(base.height);
   const double fscale = std::ldexp(1., int(finest)), fphase = (fscale - 1) * .5;
   ImageView fine{lev[finest].v, lw[finest], lh[finest]};
   if ((type == 1 ? 65535.0 : 255.0) * std::ldexp(1., int(2 * finest)) <= 2048.0) {
@@ -1884,24 +1890,21 @@ FindOutput run_find(mvg_ncc_model_s& m, const void* pixels, int type, int64_t W,
       Span sp(kStScore, s);
       check(launch_score(sa, cap, s), "score");
     }
+    ws.sort_keys.reserve(2 * size_t(cap));
+    ws.sort_idx.reserve(2 * size_t(cap));
     SortArgs so;
     so.in = cur;
     so.out = ws.sorted.p;
     so.state = st;
     so.slot = slot;
-    so.keys = nullptr;
-    so.idx = nullptr;
-    so.npow = 0;
-    if (cap > kRankSortMax) {
-      int np = 4096;
-      while (np < cap) np <<= 1;
-      ws.sort_keys.reserve(size_t(np));
-      ws.sort_idx.reserve(size_t(np));
-      so.keys = ws.sort_keys.p;
-      so.idx = ws.sort_idx.p;
-      so.npow = np;
-    }
-    Span sp(kStSort, s);
+    so.keys = ws.sort_keys.p;
+    so.idx = ws.sort_idx.p;
+    so.aux = prep ? nullptr : ws.aux.p;
+    so.refined_flag = ws.refined_flag.p;
+    so.tested = ws.tested.p;
+    so.sup = ws.sup.p;
+    so.geom = geom;
+    Span sp(kStSort, s, sort_launches(cap));
     check(launch_sort(so, cap, s), "sort");
   }
   if (stage == 100) {
@@ -1910,18 +1913,9 @@ FindOutput run_find(mvg_ncc_model_s& m, const void* pixels, int type, int64_t W,
   }
 
   // greedy selection with refinement (matcher.cpp:1063-1076)
-  check(cudaMemsetAsync(ws.refined_flag.p, 0, sizeof(int32_t) * size_t(cap), s), "memset");
-  check(cudaMemsetAsync(ws.tested.p, 0, sizeof(int32_t) * size_t(cap), s), "memset");
-  check(cudaMemsetAsync(ws.sup.p, 0, size_t(cap), s), "memset");
   // speculative refinement batch: the next NumMatches unsuppressed,
   // mutually non-overlapping candidates (32 when all matches are wanted)
   const int batch_limit = int(std::min<int64_t>(64, opt.num_matches > 0 ? opt.num_matches : 32));
-  RectGeom geom;
-  geom.left = -base.ocol - .5;
-  geom.right = double(base.width) - base.ocol - .5;
-  geom.top = -base.orow - .5;
-  geom.bottom = double(base.height) - base.orow - .5;
-  geom.area = double(base.width) * double(base.height);
   SelectArgs se;
   se.sorted = ws.sorted.p;
   se.aux = ws.aux.p;
@@ -2017,8 +2011,7 @@ FindOutput run_find(mvg_ncc_model_s& m, const void* pixels, int type, int64_t W,
     return out;
   }
   {
-    Span sp(kStSelect, s, 2);
-    check(launch_rects(ws.sorted.p, ws.aux.p, st, geom, cap, s), "rects");
+    Span sp(kStSelect, s);
     check(launch_select(se, s), "select");
   }
   // A round that accepts nothing (the candidates fail refinement or overlap)

@@ -1592,83 +1592,17 @@ __device__ __forceinline__ unsigned long long desc_key(double s) {
   return ~asc;
 }
 
-// Rank sort: the output position of a candidate is the number of candidates
-// before it in the reference's order (score descending, then row, column,
-// angle; matcher.cpp:824-827).  Poses are unique after the merge, so the
-// ranks are a permutation.  A block ranks 64 candidates, four threads each
-// counting over a quarter of every 2048-key tile of the list in shared
-// memory; pose ties (equal keys) read the poses from global memory.
-constexpr int kSortPer = 64;
-__global__ void __launch_bounds__(256) sort_kernel(SortArgs a) {
-  __shared__ unsigned long long s_key[2048];
-  __shared__ int s_finite;
-  const int n = live_count(a.state, a.slot);
-  if (int(blockIdx.x) * kSortPer >= n) return;
-  if (a.keys && n > kRankSortMax) return;  // the bitonic sort takes it
-  const int lane4 = threadIdx.x & 3;
-  const int i = blockIdx.x * kSortPer + (threadIdx.x >> 2);
-  Cand me{};
-  unsigned long long key = ~0ULL;
-  if (i < n) {
-    me = a.in[i];
-    key = desc_key(me.score);
-  }
-  if (threadIdx.x == 0) s_finite = 0;
-  int rank = 0;
-  for (int base = 0; base < n; base += 2048) {
-    const int m = min(2048, n - base);
-    __syncthreads();
-    for (int k = threadIdx.x; k < m; k += 256) s_key[k] = desc_key(a.in[base + k].score);
-    __syncthreads();
-    if (i < n) {
-      int r0 = 0, r1 = 0;
-      int k = lane4;
-      for (; k + 4 < m; k += 8) {
-        const unsigned long long k0 = s_key[k], k1 = s_key[k + 4];
-        r0 += k0 < key;
-        r1 += k1 < key;
-        if (k0 == key || k1 == key) {
-          for (int q = 0; q < 2; ++q) {
-            const int kk = k + 4 * q;
-            if (s_key[kk] != key) continue;
-            const Cand c = a.in[base + kk];
-            if (c.row < me.row || (c.row == me.row && (c.col < me.col || (c.col == me.col && c.angle < me.angle))))
-              ++r0;
-          }
-        }
-      }
-      for (; k < m; k += 4) {
-        const unsigned long long k0 = s_key[k];
-        r0 += k0 < key;
-        if (k0 == key) {
-          const Cand c = a.in[base + k];
-          if (c.row < me.row || (c.row == me.row && (c.col < me.col || (c.col == me.col && c.angle < me.angle))))
-            ++r0;
-        }
-      }
-      rank += r0 + r1;
-    }
-  }
-  rank += __shfl_xor_sync(0xffffffffu, rank, 1);
-  rank += __shfl_xor_sync(0xffffffffu, rank, 2);
-  if (i < n && lane4 == 0) {
-    a.out[rank] = me;
-    if (isfinite(me.score)) atomicAdd(&s_finite, 1);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0 && s_finite) atomicAdd(&a.state->sorted_count, s_finite);
-}
+// Candidate sort in the reference's order (score descending, then row,
+// column, angle; matcher.cpp:824-827; the list index for exact duplicates):
+// 256-entry segments are ranked in shared memory, then an entry's place among
+// up to 64 sorted lists is its place in its own plus the entries of every
+// other list before it (binary search).  One merge covers 16384 candidates,
+// two 2^20, three 2^26; every launch reads the live count and returns when
+// the list is already sorted.  Bound by the latency of the searches.
+constexpr int kSortSeg = 256, kSortFan = 64, kSortLanes = 8;
 
-// Bitonic sort of long candidate lists (more than kRankSortMax): (key,
-// index) pairs, padded to the power of two at or above the live count with
-// entries that order after every candidate; the comparator is the rank
-// sort's order (descending score key, then row, column, angle; the index for
-// exact duplicates).  Stages with k up to 2048 and the j < 2048 steps of
-// longer stages run in shared memory, one 2048-entry segment per block.
 __device__ __forceinline__ bool sort_before(unsigned long long ka, int ia, unsigned long long kb, int ib,
                                             const Cand* __restrict__ in) {
-  if (ia == INT32_MAX) return false;
-  if (ib == INT32_MAX) return true;
   if (ka != kb) return ka < kb;
   const Cand x = in[ia], y = in[ib];
   if (x.row != y.row) return x.row < y.row;
@@ -1677,106 +1611,111 @@ __device__ __forceinline__ bool sort_before(unsigned long long ka, int ia, unsig
   return ia < ib;
 }
 
-__device__ __forceinline__ int bitonic_live(const SortArgs& a) {
-  const int n = live_count(a.state, a.slot);
-  if (n <= kRankSortMax) return 0;
-  int p = 1;
-  while (p < n) p <<= 1;
-  return p;
+__device__ RectAux make_rect(const Cand& m, const RectGeom& g);
+
+// Candidate i at its final rank, and the selection's per-candidate state.
+__device__ __forceinline__ bool sort_emit(const SortArgs& a, int rank, int i) {
+  const Cand c = a.in[i];
+  a.out[rank] = c;
+  if (a.aux) {
+    a.aux[rank] = make_rect(c, a.geom);
+    a.refined_flag[rank] = 0;
+    a.tested[rank] = 0;
+    a.sup[rank] = 0;
+  }
+  return isfinite(c.score);
 }
 
-__global__ void __launch_bounds__(256) bitonic_init_kernel(SortArgs a) {
-  const int np = bitonic_live(a);
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= np) return;
+__global__ void __launch_bounds__(kSortSeg) sort_segments_kernel(SortArgs a) {
+  __shared__ __align__(16) unsigned long long s_key[kSortSeg];
   const int n = live_count(a.state, a.slot);
-  a.keys[r] = r < n ? desc_key(a.in[r].score) : ~0ULL;
-  a.idx[r] = r < n ? r : INT32_MAX;
-}
-
-// all steps j <= min(k, 2048) / 2 of the stages k0 .. k1 (k0 <= k1 <= 2048:
-// the whole network up to 2048; k0 == k1 > 2048: the shared-memory tail of
-// one stage) on this block's 2048-entry segment
-__global__ void __launch_bounds__(1024) bitonic_block_kernel(SortArgs a, int k0, int k1) {
-  __shared__ unsigned long long s_key[2048];
-  __shared__ int s_idx[2048];
-  const int np = bitonic_live(a);
-  const int base = blockIdx.x * 2048;
-  if (base >= np || k0 > np) return;
-  const int t = threadIdx.x;
-  s_key[t] = a.keys[base + t];
-  s_idx[t] = a.idx[base + t];
-  s_key[t + 1024] = a.keys[base + t + 1024];
-  s_idx[t + 1024] = a.idx[base + t + 1024];
+  const int base = blockIdx.x * kSortSeg, t = threadIdx.x, i = base + t;
+  if (base >= n) return;
+  const unsigned long long key = i < n ? desc_key(a.in[i].score) : ~0ULL;
+  s_key[t] = key;
   __syncthreads();
-  for (int k = k0; k <= k1; k <<= 1) {
-    for (int j = min(k, 2048) >> 1; j > 0; j >>= 1) {
-      const int i = ((t & ~(j - 1)) << 1) | (t & (j - 1)), l = i + j;
-      const bool up = ((base + i) & k) == 0;
-      const unsigned long long ki = s_key[i], kl = s_key[l];
-      const int ii = s_idx[i], il = s_idx[l];
-      if (sort_before(kl, il, ki, ii, a.in) == up) {
-        s_key[i] = kl;
-        s_key[l] = ki;
-        s_idx[i] = il;
-        s_idx[l] = ii;
-      }
-      __syncthreads();
+  int rank = 0;
+  bool tie = false;
+#pragma unroll 8
+  for (int k = 0; k < kSortSeg; k += 2) {
+    const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(s_key + k);
+    rank += int(q.x < key) + int(q.y < key);
+    tie |= (q.x == key && k != t) || (q.y == key && k + 1 != t);
+  }
+  if (tie && i < n)
+    for (int k = 0; k < min(kSortSeg, n - base); ++k)
+      rank += k != t && s_key[k] == key && sort_before(key, base + k, key, i, a.in);
+  bool finite = false;
+  if (i < n) {
+    if (n > kSortSeg) {
+      a.keys[base + rank] = key;
+      a.idx[base + rank] = i;
+    } else {
+      finite = sort_emit(a, rank, i);
     }
   }
-  a.keys[base + t] = s_key[t];
-  a.idx[base + t] = s_idx[t];
-  a.keys[base + t + 1024] = s_key[t + 1024];
-  a.idx[base + t + 1024] = s_idx[t + 1024];
+  const unsigned m = __ballot_sync(0xffffffffu, finite);
+  if ((t & 31) == 0 && m) atomicAdd(&a.state->sorted_count, __popc(m));
 }
 
-// one step j >= 2048 of stage k, in global memory
-__global__ void __launch_bounds__(256) bitonic_step_kernel(SortArgs a, int k, int j) {
-  const int np = bitonic_live(a);
-  if (k > np) return;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (np >> 1)) return;
-  const int i = ((t & ~(j - 1)) << 1) | (t & (j - 1)), l = i + j;
-  const bool up = (i & k) == 0;
-  const unsigned long long ki = a.keys[i], kl = a.keys[l];
-  const int ii = a.idx[i], il = a.idx[l];
-  if (sort_before(kl, il, ki, ii, a.in) == up) {
-    a.keys[i] = kl;
-    a.keys[l] = ki;
-    a.idx[i] = il;
-    a.idx[l] = ii;
-  }
-}
-
-__global__ void __launch_bounds__(256) bitonic_gather_kernel(SortArgs a) {
-  __shared__ int s_finite;
-  const int np = bitonic_live(a);
-  if (!np) return;
+// Merges groups of kSortFan sorted segments of `seg` entries (eight threads
+// per entry share the group's segments).
+__global__ void __launch_bounds__(256) sort_merge_kernel(SortArgs a, int seg, const unsigned long long* __restrict__ keys,
+                                                         const int32_t* __restrict__ idx, unsigned long long* keys_out,
+                                                         int32_t* idx_out) {
   const int n = live_count(a.state, a.slot);
-  if (threadIdx.x == 0) s_finite = 0;
-  __syncthreads();
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r < n) {
-    const Cand c = a.in[a.idx[r]];
-    a.out[r] = c;
-    if (isfinite(c.score)) atomicAdd(&s_finite, 1);
+  if (n <= seg) return;
+  const int sub = threadIdx.x % kSortLanes;
+  const int e = int((blockIdx.x * 256u + threadIdx.x) / kSortLanes);
+  bool finite = false;
+  const long long span = (long long)seg * kSortFan;
+  const int group = int(e / span) * kSortFan, own = e / seg;  // first segment of the group; the entry's segment
+  int rank = 0;
+  if (e < n) {
+    const unsigned long long key = keys[e];
+    const int i = idx[e];
+    for (int t = group + sub; t < group + kSortFan && (long long)t * seg < n; t += kSortLanes) {
+      if (t == own) continue;
+      const int first = t * seg;
+      int lo = 0, hi = min(seg, n - first);
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (sort_before(keys[first + mid], idx[first + mid], key, i, a.in))
+          lo = mid + 1;
+        else
+          hi = mid;
+      }
+      rank += lo;
+    }
   }
-  __syncthreads();
-  if (threadIdx.x == 0 && s_finite) atomicAdd(&a.state->sorted_count, s_finite);
+#pragma unroll
+  for (int o = 1; o < kSortLanes; o <<= 1) rank += __shfl_xor_sync(0xffffffffu, rank, o);
+  if (e < n && sub == 0) {
+    rank += group * seg + (e - own * seg);
+    if (n <= span) {
+      finite = sort_emit(a, rank, idx[e]);
+    } else {
+      keys_out[rank] = keys[e];
+      idx_out[rank] = idx[e];
+    }
+  }
+  const unsigned m = __ballot_sync(0xffffffffu, finite);
+  if ((threadIdx.x & 31) == 0 && m) atomicAdd(&a.state->sorted_count, __popc(m));
 }
 
 // ----------------------------------------------------------------- overlap
-// Rotated rectangle of a pose: FP64 cos/sin once per pose, a conservative
-// FP32 box for the cheap disjointness test.
+// Rotated rectangle of a pose: FP32 cos/sin and a conservative FP32 box for
+// the cheap disjointness test.  FP64 sincos is left to the exact overlap,
+// which few pairs need: one per sorted candidate took 18 us of a small find.
 __device__ RectAux make_rect(const Cand& m, const RectGeom& g) {
   RectAux r;
-  sincos(m.angle, &r.sa, &r.ca);
+  sincosf(float(m.angle), &r.sa, &r.ca);
   float x0 = INFINITY, y0 = INFINITY, x1 = -INFINITY, y1 = -INFINITY;
   const double xs[2] = {g.left, g.right}, ys[2] = {g.top, g.bottom};
   for (double x : xs)
     for (double y : ys) {
-      const float px = float(m.col) + float(r.ca) * float(x) + float(r.sa) * float(y);
-      const float py = float(m.row) - float(r.sa) * float(x) + float(r.ca) * float(y);
+      const float px = float(m.col) + r.ca * float(x) + r.sa * float(y);
+      const float py = float(m.row) - r.sa * float(x) + r.ca * float(y);
       x0 = fminf(x0, px);
       x1 = fmaxf(x1, px);
       y0 = fminf(y0, py);
@@ -1803,13 +1742,16 @@ struct Pt {
 // accepted match.  Corners are relative to a's centre.
 __device__ double overlap_ratio(const Cand& a, const RectAux& ra, const Cand& b, const RectAux& rb, const RectGeom& g) {
   if (boxes_disjoint(ra, rb)) return 0.;
+  double aca, asa, bca, bsa;
+  sincos(a.angle, &asa, &aca);
+  sincos(b.angle, &bsa, &bca);
   const Pt in[4] = {{g.left, g.top}, {g.right, g.top}, {g.right, g.bottom}, {g.left, g.bottom}};
   Pt clip[4], poly[16], next[16];
   for (int i = 0; i < 4; ++i) {
-    clip[i].x = dadd(dadd(dsub(b.col, a.col), dmul(rb.ca, in[i].x)), dmul(rb.sa, in[i].y));
-    clip[i].y = dadd(dsub(dsub(b.row, a.row), dmul(rb.sa, in[i].x)), dmul(rb.ca, in[i].y));
-    poly[i].x = dadd(dmul(ra.ca, in[i].x), dmul(ra.sa, in[i].y));
-    poly[i].y = dadd(-dmul(ra.sa, in[i].x), dmul(ra.ca, in[i].y));
+    clip[i].x = dadd(dadd(dsub(b.col, a.col), dmul(bca, in[i].x)), dmul(bsa, in[i].y));
+    clip[i].y = dadd(dsub(dsub(b.row, a.row), dmul(bsa, in[i].x)), dmul(bca, in[i].y));
+    poly[i].x = dadd(dmul(aca, in[i].x), dmul(asa, in[i].y));
+    poly[i].y = dadd(-dmul(asa, in[i].x), dmul(aca, in[i].y));
   }
   int count = 4;
   for (int edge = 0; edge < 4 && count; ++edge) {
@@ -1841,7 +1783,7 @@ __device__ float overlap_ratio32(const Cand& a, const RectAux& ra, const Cand& b
   const float L = float(g.left), R = float(g.right), T = float(g.top), B = float(g.bottom);
   const float inx[4] = {L, R, R, L}, iny[4] = {T, T, B, B};
   const float dx = float(b.col - a.col), dy = float(b.row - a.row);
-  const float bca = float(rb.ca), bsa = float(rb.sa), aca = float(ra.ca), asa = float(ra.sa);
+  const float bca = rb.ca, bsa = rb.sa, aca = ra.ca, asa = ra.sa;
   float cx[4], cy[4], px[16], py[16], nx[16], ny[16];
   for (int i = 0; i < 4; ++i) {
     cx[i] = dx + bca * inx[i] + bsa * iny[i];
@@ -1887,12 +1829,6 @@ __device__ __forceinline__ bool overlaps(const Cand& a, const RectAux& ra, const
   if (double(r32) > thr + 1e-3) return true;
   if (double(r32) < thr - 1e-3) return false;
   return overlap_ratio(a, ra, b, rb, g) > thr;
-}
-
-__global__ void rects_kernel(const Cand* sorted, RectAux* aux, const QueryState* state, RectGeom g) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= state->sorted_count) return;
-  aux[i] = make_rect(sorted[i], g);
 }
 
 // Greedy MaxOverlap selection over the sorted candidates
@@ -2638,26 +2574,20 @@ cudaError_t launch_pairs(const float* v, int w, int h, uint32_t* pairs, cudaStre
 }
 
 cudaError_t launch_sort(const SortArgs& a, int max_candidates, cudaStream_t s) {
-  sort_kernel<<<(max_candidates + kSortPer - 1) / kSortPer, 256, 0, s>>>(a);
-  if (a.keys) {
-    // every launch reads the live count and returns when it has no work
-    if (a.npow < max_candidates || a.npow < 4096 || (a.npow & (a.npow - 1))) return cudaErrorInvalidValue;
-    const unsigned segs = unsigned(a.npow / 2048), pairs = unsigned(a.npow / 2 / 256);
-    bitonic_init_kernel<<<unsigned(a.npow / 256), 256, 0, s>>>(a);
-    bitonic_block_kernel<<<segs, 1024, 0, s>>>(a, 2, 2048);
-    for (int k = 4096; k <= a.npow; k <<= 1) {
-      for (int j = k >> 1; j >= 2048; j >>= 1) bitonic_step_kernel<<<pairs, 256, 0, s>>>(a, k, j);
-      bitonic_block_kernel<<<segs, 1024, 0, s>>>(a, k, k);
-    }
-    bitonic_gather_kernel<<<unsigned((max_candidates + 255) / 256), 256, 0, s>>>(a);
+  sort_segments_kernel<<<(max_candidates + kSortSeg - 1) / kSortSeg, kSortSeg, 0, s>>>(a);
+  const unsigned blocks = unsigned(((long long)max_candidates * kSortLanes + 255) / 256);
+  int from = 0;  // lists alternate between the two halves of keys / idx
+  for (long long seg = kSortSeg; seg < max_candidates; seg *= kSortFan, from ^= 1) {
+    const size_t in = from ? max_candidates : 0, out = from ? 0 : max_candidates;
+    sort_merge_kernel<<<blocks, 256, 0, s>>>(a, int(seg), a.keys + in, a.idx + in, a.keys + out, a.idx + out);
   }
   return cudaGetLastError();
 }
 
-cudaError_t launch_rects(const Cand* sorted, RectAux* aux, const QueryState* state, RectGeom g, int max_candidates,
-                         cudaStream_t s) {
-  rects_kernel<<<unsigned((max_candidates + 255) / 256), 256, 0, s>>>(sorted, aux, state, g);
-  return cudaGetLastError();
+int sort_launches(int max_candidates) {
+  int n = 1;
+  for (long long seg = kSortSeg; seg < max_candidates; seg *= kSortFan) ++n;
+  return n;
 }
 
 cudaError_t launch_select(const SelectArgs& a, cudaStream_t s) {

@@ -306,12 +306,15 @@ struct Refine4Args {
   double max_shift, max_angle, max_scale;  // step limits per iteration
 };
 
-// Candidate sort.  Lists of up to kRankSortMax candidates are rank-sorted
-// in one launch; longer ones (candidate budgets above it) by a bitonic sort
-// of (key, index) pairs in `keys` / `idx` (npow entries each, npow the power
-// of two at or above the budget; null when the budget is at most
-// kRankSortMax).  Both give the same order.
-constexpr int kRankSortMax = 16384;
+// Level-0 model rectangle about the origin: [left, right] x [top, bottom]
+// (src/ncc_matching/matcher.cpp:257-258).
+struct RectGeom {
+  double left, right, top, bottom, area;
+};
+
+// Candidate sort (score descending, then row, column, angle).  keys / idx:
+// twice the candidate budget each.  With aux, every sorted candidate also gets
+// its rectangle and cleared selection state.
 struct SortArgs {
   const Cand* in;
   Cand* out;
@@ -319,13 +322,11 @@ struct SortArgs {
   int slot;
   unsigned long long* keys;
   int32_t* idx;
-  int npow;
-};
-
-// Level-0 model rectangle about the origin: [left, right] x [top, bottom]
-// (src/ncc_matching/matcher.cpp:257-258).
-struct RectGeom {
-  double left, right, top, bottom, area;
+  RectAux* aux;             // nullable
+  int32_t* refined_flag;
+  int32_t* tested;
+  uint8_t* sup;
+  RectGeom geom;
 };
 
 // Refinement / selection
@@ -381,8 +382,7 @@ cudaError_t launch_score(const ScoreArgs& a, int max_candidates, cudaStream_t s)
 cudaError_t launch_adjoint(const AdjointArgs& a, cudaStream_t s);
 cudaError_t launch_refine4(const Refine4Args& a, cudaStream_t s);
 cudaError_t launch_sort(const SortArgs& a, int max_candidates, cudaStream_t s);
-cudaError_t launch_rects(const Cand* sorted, RectAux* aux, const QueryState* state, RectGeom g, int max_candidates,
-                         cudaStream_t s);
+int sort_launches(int max_candidates);  // kernels launch_sort queues
 cudaError_t launch_select(const SelectArgs& a, cudaStream_t s);
 cudaError_t launch_refine(const RefineArgs& a, int batch_limit, cudaStream_t s);
 

@@ -75,10 +75,10 @@ struct Cand {
   int32_t pad;
 };
 
-// Rotated template rectangle of a pose for the MaxOverlap test: FP64 cos/sin
+// Rotated template rectangle of a pose for the MaxOverlap test: FP32 cos/sin
 // and a conservative FP32 axis-aligned box in image coordinates.
 struct RectAux {
-  double ca, sa;
+  float ca, sa;
   float x0, y0, x1, y1;
 };
 
