@@ -1883,12 +1883,12 @@ FindOutput run_find(mvg_ncc_model_s& m, const void* pixels, int type, int64_t W,
     sa.slot = slot;
     sa.crop_row = double(crop_row);
     sa.crop_col = double(crop_col);
-    sa.scale = fscale;
     sa.phase = fphase;
+    sa.inv_scale = 1 / fscale;
     sa.absolute = hm.params.ignore_polarity;
     {
       Span sp(kStScore, s);
-      check(launch_score(sa, cap, s), "score");
+      check(launch_score(sa, cap, s, ws.sm_count), "score");
     }
     ws.sort_keys.reserve(2 * size_t(cap));
     ws.sort_idx.reserve(2 * size_t(cap));
@@ -1949,6 +1949,7 @@ FindOutput run_find(mvg_ncc_model_s& m, const void* pixels, int type, int64_t W,
   ra.crop_col = double(crop_col);
   ra.scale = fscale;
   ra.phase = fphase;
+  ra.inv_scale = 1 / fscale;
   ra.angle_start = opt.angle_start;
   ra.angle_end = opt.angle_start + opt.angle_extent;
   ra.angle_step = hm.params.angle_step;

@@ -1072,34 +1072,58 @@ __global__ void dedup_kernel(DedupArgs a) {
 }
 
 // -------------------------------------------------- full-resolution scoring
-// Totals of K per-thread values as FP32 pairs; valid on thread 0 only.
-// scratch: K*64 floats.
-template <int K>
-__device__ void block_total(const float (&v)[K], F2 (&out)[K], float* scratch) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+// Block totals of K per-thread values as FP32 pairs, in s.total[k] for every
+// thread.  The order of the additions is that of a shuffle tree over the
+// lanes (16, 8, 4, 2, 1 apart) and one over the warps, but a lane carries
+// only the values it will own: each step halves them, so 19 values cost 21
+// pair additions a lane instead of 95, and the warps' partials are added by
+// one warp per value instead of one warp for all.  (Pair addition is
+// commutative to the bit, and adding a zero pair changes nothing.)
+template <int K> struct BlockTotals {
+  F2 part[K][16];  // by value and warp
+  F2 total[K];
+};
+
+template <int N> struct LaneFold {
+  // x: N values of which this lane's subset holds `count`; halves them
+  static __device__ __forceinline__ F2 run(const F2 (&x)[N], int bit, int& index, int& count) {
+    constexpr int H = (N + 1) / 2;
+    const bool up = threadIdx.x & bit;
+    F2 y[H];
 #pragma unroll
-  for (int k = 0; k < K; ++k) {
-    F2 x = f2(v[k]);
-    for (int o = 16; o > 0; o >>= 1) {
-      const F2 y{__shfl_down_sync(0xffffffffu, x.hi, o), __shfl_down_sync(0xffffffffu, x.lo, o)};
-      x = f2_add(x, y);
+    for (int i = 0; i < H; ++i) {
+      const F2 a = x[i], b = i + H < N ? x[i + H < N ? i + H : 0] : F2{0.f, 0.f};
+      const F2 send = up ? a : b, keep = up ? b : a;
+      y[i] = f2_add(keep, F2{__shfl_xor_sync(0xffffffffu, send.hi, bit), __shfl_xor_sync(0xffffffffu, send.lo, bit)});
     }
-    if (lane == 0) {
-      scratch[(k * 32 + warp) * 2] = x.hi;
-      scratch[(k * 32 + warp) * 2 + 1] = x.lo;
-    }
+    index += up ? H : 0;
+    count = up ? count - H : min(count, H);
+    return LaneFold<H>::run(y, bit >> 1, index, count);
   }
-  __syncthreads();
-  if (warp == 0) {
+};
+template <> struct LaneFold<1> {
+  static __device__ __forceinline__ F2 run(const F2 (&x)[1], int bit, int&, int&) {
+    F2 y = x[0];
+    for (; bit > 0; bit >>= 1)
+      y = f2_add(y, F2{__shfl_xor_sync(0xffffffffu, y.hi, bit), __shfl_xor_sync(0xffffffffu, y.lo, bit)});
+    return y;
+  }
+};
+
+template <int K> __device__ __forceinline__ void block_total(const float (&v)[K], BlockTotals<K>& s) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  F2 x[K];
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      F2 y = lane < nw ? F2{scratch[(k * 32 + lane) * 2], scratch[(k * 32 + lane) * 2 + 1]} : F2{0.f, 0.f};
-      for (int o = 16; o > 0; o >>= 1) {
-        const F2 z{__shfl_down_sync(0xffffffffu, y.hi, o), __shfl_down_sync(0xffffffffu, y.lo, o)};
-        y = f2_add(y, z);
-      }
-      out[k] = y;
-    }
+  for (int k = 0; k < K; ++k) x[k] = f2(v[k]);
+  int index = 0, count = K;
+  const F2 mine = LaneFold<K>::run(x, 16, index, count);
+  if (count > 0) s.part[index][warp] = mine;
+  __syncthreads();
+  for (int k = warp; k < K; k += nw) {
+    F2 y = lane < nw ? s.part[k][lane] : F2{0.f, 0.f};
+    for (int o = nw >> 1; o > 0; o >>= 1)
+      y = f2_add(y, F2{__shfl_down_sync(0xffffffffu, y.hi, o), __shfl_down_sync(0xffffffffu, y.lo, o)});
+    if (lane == 0) s.total[k] = y;
   }
   __syncthreads();
 }
@@ -1111,15 +1135,20 @@ struct LocalPose {
   float ca, sa;
 };
 
-__device__ __forceinline__ LocalPose make_local(double row, double col, double angle) {
-  LocalPose l;
-  const double fr = floor(row), fc = floor(col);
-  l.R0 = int(fr);
-  l.C0 = int(fc);
-  l.fr = float(row - fr);
-  l.fc = float(col - fc);
-  sincosf(float(angle), &l.sa, &l.ca);
-  return l;
+// Level-local pose of a pose in image coordinates, by lanes 0 to 2 of a warp
+// (row, column, angle side by side: FP64 latencies once).  The level scale is
+// a power of two, so multiplying by its inverse divides exactly.
+__device__ __forceinline__ void set_local(LocalPose& l, const double* pose, double crop_row, double crop_col,
+                                          double phase, double inv_scale) {
+  const int lane = threadIdx.x & 31;
+  if (lane < 2) {
+    const double v = (pose[lane] - (lane ? crop_col : crop_row) - phase) * inv_scale;
+    const double f = floor(v);
+    (lane ? l.C0 : l.R0) = int(f);
+    (lane ? l.fc : l.fr) = float(v - f);
+  } else if (lane == 2) {
+    sincosf(float(pose[2]), &l.sa, &l.ca);
+  }
 }
 
 // True when every sample of the rotated original lies inside the image by a
@@ -1144,20 +1173,18 @@ __device__ __forceinline__ bool samples_inside(const LocalPose& L, const Origina
   return y0 >= hmin + m && x0 >= wmin + m && y1 <= hmax - 1.f - m && x1 <= wmax - 1.f - m;
 }
 
-// Shared state of a block working on one pose at a time.
-struct PoseShared {
-  LocalPose lp;
-  double score;       // result of the last continuous pass
-  int ok;             // result flag of the last Gauss-Newton pass
-  double gscore;      // score seen by the last Gauss-Newton pass (-inf if none)
-  double delta[3];
-  float scratch[19 * 64];
-};
-
 __device__ __forceinline__ float bilinear_at(const ImageView& img, int r, int c, float fy, float fx, int r1, int c1) {
   const float* v = img.v;
   return (1 - fy) * ((1 - fx) * __ldg(v + size_t(r) * img.w + c) + fx * __ldg(v + size_t(r) * img.w + c1)) +
          fy * ((1 - fx) * __ldg(v + size_t(r1) * img.w + c) + fx * __ldg(v + size_t(r1) * img.w + c1));
+}
+
+// Integer part (towards minus infinity) and fraction of |v| < 2^22, without
+// the conversion unit: v + 1.5 * 2^23 rounded down is floor(v) + 1.5 * 2^23.
+__device__ __forceinline__ int split_floor(float v, float& frac) {
+  const float t = __fadd_rd(v, 12582912.f);
+  frac = v - __fsub_rn(t, 12582912.f);
+  return __float_as_int(t) - 0x4b400000;
 }
 
 // FP32 score from pair totals of sum q, sum q^2, sum w q.
@@ -1171,12 +1198,10 @@ __device__ __forceinline__ float pair_score(F2 sum, F2 sq, F2 dot, int n, int ab
 }
 
 // continuous() of src/ncc_matching/matcher.cpp:144-156 at a level-local pose;
-// every thread of the block calls it; sh.score holds the result afterwards.
-__device__ void continuous_pass(const ImageView& img, const OriginalView& orig, double row, double col, double angle,
-                                int absolute, PoseShared& sh) {
-  if (threadIdx.x == 0) sh.lp = make_local(row, col, angle);
-  __syncthreads();
-  const LocalPose L = sh.lp;
+// every thread of the block calls it and gets the score.
+__device__ __forceinline__ double continuous_pass(const ImageView& img, const OriginalView& orig, const LocalPose& lp,
+                                                  int absolute, BlockTotals<4>& tot) {
+  const LocalPose L = lp;
   const float hmax = float(img.h - 1 - L.R0), wmax = float(img.w - 1 - L.C0);
   const float hmin = float(-L.R0), wmin = float(-L.C0);
   float offset = 0.f;
@@ -1210,9 +1235,7 @@ __device__ void continuous_pass(const ImageView& img, const OriginalView& orig, 
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const float y = L.fr + (L.ca * p[u].x - L.sa * p[u].y), x = L.fc + (L.sa * p[u].x + L.ca * p[u].y);
-        const int iy = __float2int_rd(y), ix = __float2int_rd(x);
-        fy[u] = y - float(iy);
-        fx[u] = x - float(ix);
+        const int iy = split_floor(y, fy[u]), ix = split_floor(x, fx[u]);
         if (pbase) {
           const uint32_t* pp = pbase + (iy * w + ix);
           const uint32_t aq = __ldg(pp), bq = __ldg(pp + w);
@@ -1253,26 +1276,27 @@ __device__ void continuous_pass(const ImageView& img, const OriginalView& orig, 
     acc[1] = fmaf(q, q, acc[1]);
     acc[2] = fmaf(w, q, acc[2]);
   }
-  F2 t[4];
-  block_total<4>(acc, t, sh.scratch);
-  if (threadIdx.x == 0) {
-    bool ok = false;
-    const float sc = t[3].hi > 0 ? -INFINITY : pair_score(t[0], t[1], t[2], orig.n, absolute, &ok);
-    sh.score = (t[3].hi > 0 || !ok) ? -INFINITY : double(sc);
-  }
-  __syncthreads();
+  block_total<4>(acc, tot);
+  bool ok = false;
+  const float sc = tot.total[3].hi > 0 ? -INFINITY
+                                       : pair_score(tot.total[0], tot.total[1], tot.total[2], orig.n, absolute, &ok);
+  return ok ? double(sc) : -INFINITY;
 }
 
 __global__ void __launch_bounds__(128, 12) score_kernel(ScoreArgs a) {
-  __shared__ PoseShared sh;
-  const int i = blockIdx.x;
-  if (i >= live_count(a.state, a.slot)) return;
-  const Cand c = a.cand[i];
-  if (!isfinite(c.score)) return;
-  const double row = (c.row - a.crop_row - a.phase) / a.scale;
-  const double col = (c.col - a.crop_col - a.phase) / a.scale;
-  continuous_pass(a.img, a.orig, row, col, c.angle, a.absolute, sh);
-  if (threadIdx.x == 0) a.cand[i].score = sh.score;
+  __shared__ BlockTotals<4> tot;
+  __shared__ LocalPose lp;
+  const int live = live_count(a.state, a.slot);
+  // candidates strided over a bounded grid: a block per possible candidate
+  // costs more than a short list's work when the budget is large
+  for (int i = blockIdx.x; i < live; i += gridDim.x) {
+    const Cand& c = a.cand[i];
+    if (!isfinite(c.score)) continue;
+    if (threadIdx.x < 32) set_local(lp, &c.row, a.crop_row, a.crop_col, a.phase, a.inv_scale);
+    __syncthreads();
+    const double score = continuous_pass(a.img, a.orig, lp, a.absolute, tot);
+    if (threadIdx.x == 0) a.cand[i].score = score;
+  }
 }
 
 // ------------------------------------------------------------- NCC adjoint
@@ -1292,7 +1316,7 @@ __global__ void __launch_bounds__(128, 12) score_kernel(ScoreArgs a) {
 constexpr int kAdjointThreads = 256;
 
 __global__ void __launch_bounds__(kAdjointThreads) adjoint_kernel(AdjointArgs a) {
-  __shared__ float scratch[17 * 64];
+  __shared__ BlockTotals<17> tot;
   __shared__ float s_off;
   const int k = blockIdx.x;
   if (k >= a.n) return;
@@ -1353,8 +1377,8 @@ __global__ void __launch_bounds__(kAdjointThreads) adjoint_kernel(AdjointArgs a)
       acc[11 + j] = fmaf(p.z, dq[j], acc[11 + j]);
     }
   }
-  F2 t[17];
-  block_total<17>(acc, t, scratch);
+  block_total<17>(acc, tot);
+  const F2* t = tot.total;
   if (threadIdx.x == 0) {
     auto dv = [](const F2& x) { return double(x.hi) + double(x.lo); };
     const double n = double(orig.n);
@@ -1453,7 +1477,7 @@ __device__ void sim_pass(const ImageView& img, const OriginalView& orig, const d
 constexpr int kRefine4Threads = 256;
 
 __global__ void __launch_bounds__(kRefine4Threads) refine4_kernel(Refine4Args a) {
-  __shared__ float scratch[kSimSums * 64];
+  __shared__ BlockTotals<kSimSums> tot;
   __shared__ float s_off;
   __shared__ double s_pose[4], s_try[4], s_delta[4], s_score, s_factor;
   __shared__ int s_go;
@@ -1463,12 +1487,12 @@ __global__ void __launch_bounds__(kRefine4Threads) refine4_kernel(Refine4Args a)
   if (threadIdx.x == 0) s_score = -INFINITY;
   __syncthreads();
   float acc[kSimSums];
-  F2 t[kSimSums];
+  const F2* t = tot.total;
   auto dv = [](const F2& x) { return double(x.hi) + double(x.lo); };
   const double n = double(a.orig.n);
   for (int it = 0; it <= a.iterations; ++it) {
     sim_pass(a.img, a.orig, s_pose, true, acc, &s_off);
-    block_total<kSimSums>(acc, t, scratch);
+    block_total<kSimSums>(acc, tot);
     if (threadIdx.x == 0) {
       s_go = 0;
       const double sq = dv(t[0]), sqq = dv(t[1]), swq = dv(t[2]), sw = dv(t[25]);
@@ -1535,7 +1559,7 @@ __global__ void __launch_bounds__(kRefine4Threads) refine4_kernel(Refine4Args a)
       if (threadIdx.x < 4) s_try[threadIdx.x] = s_pose[threadIdx.x] + ldexp(s_factor, -bt) * s_delta[threadIdx.x];
       __syncthreads();
       sim_pass(a.img, a.orig, s_try, false, acc, &s_off);
-      block_total<kSimSums>(acc, t, scratch);
+      block_total<kSimSums>(acc, tot);
       if (threadIdx.x == 0) {
         const double sq = dv(t[0]), sqq = dv(t[1]), swq = dv(t[2]), sw = dv(t[25]);
         const double E = sqq - sq * sq / n, D = swq - sq / n * sw;
@@ -1561,7 +1585,7 @@ __global__ void __launch_bounds__(kRefine4Threads) refine4_kernel(Refine4Args a)
     if (!s_go) {
       // converged: the score at the final pose
       sim_pass(a.img, a.orig, s_pose, false, acc, &s_off);
-      block_total<kSimSums>(acc, t, scratch);
+      block_total<kSimSums>(acc, tot);
       if (threadIdx.x == 0) {
         const double sq = dv(t[0]), sqq = dv(t[1]), swq = dv(t[2]), sw = dv(t[25]);
         const double E = sqq - sq * sq / n, D = swq - sq / n * sw;
@@ -1600,10 +1624,12 @@ __device__ __forceinline__ unsigned long long desc_key(double s) {
 // two 2^20, three 2^26; every launch reads the live count and returns when
 // the list is already sorted.  Bound by the latency of the searches.
 constexpr int kSortSeg = 256, kSortFan = 64, kSortLanes = 8;
+constexpr unsigned long long kNoScoreKey = 0xfff0000000000000ULL;  // desc_key(-inf)
 
 __device__ __forceinline__ bool sort_before(unsigned long long ka, int ia, unsigned long long kb, int ib,
                                             const Cand* __restrict__ in) {
   if (ka != kb) return ka < kb;
+  if (ka >= kNoScoreKey) return ia < ib;  // without a score: the order is not read
   const Cand x = in[ia], y = in[ib];
   if (x.row != y.row) return x.row < y.row;
   if (x.col != y.col) return x.col < y.col;
@@ -1634,17 +1660,18 @@ __global__ void __launch_bounds__(kSortSeg) sort_segments_kernel(SortArgs a) {
   const unsigned long long key = i < n ? desc_key(a.in[i].score) : ~0ULL;
   s_key[t] = key;
   __syncthreads();
+  const int m = min(kSortSeg, n - base);
   int rank = 0;
-  bool tie = false;
+  bool tie = false;  // another candidate has the same score
 #pragma unroll 8
-  for (int k = 0; k < kSortSeg; k += 2) {
+  for (int k = 0; k < m; k += 2) {
     const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(s_key + k);
-    rank += int(q.x < key) + int(q.y < key);
+    rank += int(q.x < key || (q.x == key && k < t)) + int(q.y < key || (q.y == key && k + 1 < t));
     tie |= (q.x == key && k != t) || (q.y == key && k + 1 != t);
   }
-  if (tie && i < n)
-    for (int k = 0; k < min(kSortSeg, n - base); ++k)
-      rank += k != t && s_key[k] == key && sort_before(key, base + k, key, i, a.in);
+  if (tie && i < n && key < kNoScoreKey)
+    for (int k = 0; k < m; ++k)
+      if (k != t && s_key[k] == key) rank += int(sort_before(key, base + k, key, i, a.in)) - int(k < t);
   bool finite = false;
   if (i < n) {
     if (n > kSortSeg) {
@@ -1971,15 +1998,33 @@ __global__ void __launch_bounds__(kSelectThreads) select_kernel(SelectArgs a) {
 }
 
 // --------------------------------------------------------------- refinement
-// refinement_step of src/ncc_matching/matcher.cpp:170-240 at a level-local
-// pose: bilinear samples with the analytic gradient, FP32 per thread, pair
+// State of a block's fit.  Poses are {row, column, angle}; scalar FP64 work
+// is done by warp 0, a pose component per lane, and read by all threads
+// after a barrier.
+struct FitShared {
+  LocalPose lp;        // pose of the next pass
+  BlockTotals<4> tot4;
+  BlockTotals<19> tot19;
+  double pose[3], trial[3], seed[3], best[3];
+  double delta[3], gn_delta[3], next_delta[3];
+  double gscore, factor;  // score seen by the last Gauss-Newton pass (-inf if none); step factor
+  int ok, flag;           // result of the last Gauss-Newton pass; a decision of warp 0
+  float wbest[32];
+  int word[32];
+  double best_score;
+};
+
+// refinement_step of src/ncc_matching/matcher.cpp:170-240 at the pose in
+// f.lp: bilinear samples with the analytic gradient, FP32 per thread, pair
 // totals, normal equations in pair arithmetic and the Gauss-Jordan solve in
-// FP64 on thread 0.  Afterwards sh.ok / sh.gscore / sh.delta hold the result.
-__device__ void gn_pass(const ImageView& img, const OriginalView& orig, double row, double col, double angle,
-                        int absolute, int rotate, bool use_minimum, double minimum, PoseShared& sh) {
-  if (threadIdx.x == 0) sh.lp = make_local(row, col, angle);
-  __syncthreads();
-  const LocalPose L = sh.lp;
+// FP64, a matrix entry per lane of warp 0.  Afterwards f.ok / f.gscore /
+// f.gn_delta hold the result, for every thread.  Kept out of line: its code
+// runs once per pass and is called from several places, and copies of it
+// would miss the instruction cache.
+__device__ __noinline__ void gn_pass(const RefineArgs& a, FitShared& f, bool use_minimum, double minimum) {
+  const ImageView& img = a.img;
+  const OriginalView& orig = a.orig;
+  const LocalPose L = f.lp;
   const float hmax = float(img.h - 1 - L.R0), wmax = float(img.w - 1 - L.C0);
   const float hmin = float(-L.R0), wmin = float(-L.C0);
   float offset = 0.f;
@@ -1998,285 +2043,296 @@ __device__ void gn_pass(const ImageView& img, const OriginalView& orig, double r
   for (int k = 0; k < 19; ++k) acc[k] = 0.f;
   const bool inside = samples_inside(L, orig, hmin, hmax, wmin, wmax);
   const float* base = img.v + (size_t(L.R0) * img.w + L.C0);
-  for (int s = threadIdx.x; s < orig.n; s += blockDim.x) {
-    const float4 p = __ldg(orig.dcw + s);
-    const float dr = p.x, dc = p.y, w = p.z;
-    const float y = L.fr + (L.ca * dr - L.sa * dc), x = L.fc + (L.sa * dr + L.ca * dc);
-    if (!inside && !(y >= hmin && x >= wmin && y < hmax && x < wmax)) {
-      acc[18] = 1.f;
-      continue;
-    }
-    const int iy = __float2int_rd(y), ix = __float2int_rd(x);
-    const float fy = y - float(iy), fx = x - float(ix);
-    float va, vb, vd, ve;
-    if (inside && img.pairs) {
-      const uint32_t* pp = img.pairs + (size_t(L.R0) * img.w + L.C0) + (iy * img.w + ix);
-      const uint32_t aq = __ldg(pp), bq = __ldg(pp + img.w);
-      va = __half2float(__ushort_as_half(aq & 0xffff));
-      vb = __half2float(__ushort_as_half(aq >> 16));
-      vd = __half2float(__ushort_as_half(bq & 0xffff));
-      ve = __half2float(__ushort_as_half(bq >> 16));
-    } else {
-      const float* v = base + (iy * img.w + ix);
-      va = __ldg(v);
-      vb = __ldg(v + 1);
-      vd = __ldg(v + img.w);
-      ve = __ldg(v + img.w + 1);
-    }
-    const float q = (1 - fy) * ((1 - fx) * va + fx * vb) + fy * ((1 - fx) * vd + fx * ve) - offset;
-    const float gy = (1 - fx) * (vd - va) + fx * (ve - vb), gx = (1 - fy) * (vb - va) + fy * (ve - vd);
-    const float g2 = gy * (-L.sa * dr - L.ca * dc) + gx * (L.ca * dr - L.sa * dc);
-    acc[0] += q;
-    acc[1] = fmaf(q, q, acc[1]);
-    acc[2] = fmaf(w, q, acc[2]);
-    acc[3] += gy;
-    acc[4] += gx;
-    acc[5] += g2;
-    acc[6] = fmaf(q, gy, acc[6]);
-    acc[7] = fmaf(q, gx, acc[7]);
-    acc[8] = fmaf(q, g2, acc[8]);
-    acc[9] = fmaf(w, gy, acc[9]);
-    acc[10] = fmaf(w, gx, acc[10]);
-    acc[11] = fmaf(w, g2, acc[11]);
-    acc[12] = fmaf(gy, gy, acc[12]);
-    acc[13] = fmaf(gx, gy, acc[13]);
-    acc[14] = fmaf(gx, gx, acc[14]);
-    acc[15] = fmaf(g2, gy, acc[15]);
-    acc[16] = fmaf(g2, gx, acc[16]);
-    acc[17] = fmaf(g2, g2, acc[17]);
-  }
-  F2 t[19];
-  block_total<19>(acc, t, sh.scratch);
-  if (threadIdx.x < 32) {
-    // totals from lane 0 to the warp; every lane evaluates the scalar terms,
-    // lane l < axes*(axes+1) one matrix/rhs entry, lane 0 the elimination
-    const int lane = threadIdx.x;
+  const uint32_t* pbase = inside && img.pairs ? img.pairs + (size_t(L.R0) * img.w + L.C0) : nullptr;
+  const int w = img.w, stride = blockDim.x;
+  // four samples per step, all loads issued before the arithmetic; each
+  // thread still adds its samples in order s, s + blockDim.x, ...
+  constexpr int U = 4;
+  for (int s0 = threadIdx.x; s0 < orig.n; s0 += U * stride) {
+    float4 p[U];
+    float fy[U], fx[U], va[U], vb[U], vd[U], ve[U];
+    bool in[U];
 #pragma unroll
-    for (int k = 0; k < 19; ++k) {
-      t[k].hi = __shfl_sync(0xffffffffu, t[k].hi, 0);
-      t[k].lo = __shfl_sync(0xffffffffu, t[k].lo, 0);
+    for (int u = 0; u < U; ++u) {
+      const int s = s0 + u * stride;
+      in[u] = s < orig.n;
+      p[u] = in[u] ? __ldg(orig.dcw + s) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const float y = L.fr + (L.ca * p[u].x - L.sa * p[u].y), x = L.fc + (L.sa * p[u].x + L.ca * p[u].y);
+      if (!inside && in[u] && !(y >= hmin && x >= wmin && y < hmax && x < wmax)) {
+        acc[18] = 1.f;
+        in[u] = false;
+      }
+      const int iy = split_floor(y, fy[u]), ix = split_floor(x, fx[u]);
+      va[u] = vb[u] = vd[u] = ve[u] = 0.f;
+      if (!in[u]) continue;
+      if (pbase) {
+        const uint32_t* pp = pbase + (iy * w + ix);
+        const uint32_t aq = __ldg(pp), bq = __ldg(pp + w);
+        va[u] = __half2float(__ushort_as_half(aq & 0xffff));
+        vb[u] = __half2float(__ushort_as_half(aq >> 16));
+        vd[u] = __half2float(__ushort_as_half(bq & 0xffff));
+        ve[u] = __half2float(__ushort_as_half(bq >> 16));
+      } else {
+        const float* v = base + (iy * w + ix);
+        va[u] = __ldg(v);
+        vb[u] = __ldg(v + 1);
+        vd[u] = __ldg(v + w);
+        ve[u] = __ldg(v + w + 1);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (!in[u]) continue;
+      const float dr = p[u].x, dc = p[u].y, wt = p[u].z;
+      const float q = (1 - fy[u]) * ((1 - fx[u]) * va[u] + fx[u] * vb[u]) +
+                      fy[u] * ((1 - fx[u]) * vd[u] + fx[u] * ve[u]) - offset;
+      const float gy = (1 - fx[u]) * (vd[u] - va[u]) + fx[u] * (ve[u] - vb[u]),
+                  gx = (1 - fy[u]) * (vb[u] - va[u]) + fy[u] * (ve[u] - vd[u]);
+      const float g2 = gy * (-L.sa * dr - L.ca * dc) + gx * (L.ca * dr - L.sa * dc);
+      acc[0] += q;
+      acc[1] = fmaf(q, q, acc[1]);
+      acc[2] = fmaf(wt, q, acc[2]);
+      acc[3] += gy;
+      acc[4] += gx;
+      acc[5] += g2;
+      acc[6] = fmaf(q, gy, acc[6]);
+      acc[7] = fmaf(q, gx, acc[7]);
+      acc[8] = fmaf(q, g2, acc[8]);
+      acc[9] = fmaf(wt, gy, acc[9]);
+      acc[10] = fmaf(wt, gx, acc[10]);
+      acc[11] = fmaf(wt, g2, acc[11]);
+      acc[12] = fmaf(gy, gy, acc[12]);
+      acc[13] = fmaf(gx, gy, acc[13]);
+      acc[14] = fmaf(gx, gx, acc[14]);
+      acc[15] = fmaf(g2, gy, acc[15]);
+      acc[16] = fmaf(g2, gx, acc[16]);
+      acc[17] = fmaf(g2, g2, acc[17]);
+    }
+  }
+  block_total<19>(acc, f.tot19);
+  if (threadIdx.x < 32) {
+    // every lane evaluates the scalar terms, lane l < axes (axes + 1) one
+    // matrix or right-hand-side entry (row l / (axes + 1)), which it carries
+    // through the elimination
+    const F2* t = f.tot19.total;
+    const int lane = threadIdx.x;
     const F2 n = f2(float(orig.n));
     const F2 sum = t[0], dot = t[2];
     const F2 energy = f2_sub(t[1], f2_div(f2_mul(sum, sum), n));
     const float ef = f2_val(energy);
     const bool scored = !(t[18].hi > 0) && ef > 0;
-    const float sign = absolute && f2_val(dot) < 0 ? -1.f : 1.f;
+    const float sign = a.absolute && f2_val(dot) < 0 ? -1.f : 1.f;
     const float sq = scored ? sqrtf(ef) : 1.f;
     const float score = sign * f2_val(dot) / sq;
     const double gscore = scored ? double(fminf(1.f, fmaxf(-1.f, score))) : -INFINITY;
     const bool solve = scored && !(use_minimum && gscore <= minimum);
-    const int axes = rotate ? 3 : 2;
-    double entry = 0;
-    if (solve && lane < axes * (axes + 1)) {
-      const int i = lane / (axes + 1), j = lane % (axes + 1);
-      const F2 gs[3] = {t[3], t[4], t[5]}, wg[3] = {t[9], t[10], t[11]};
-      const F2 gg[3][3] = {{t[12], t[13], t[15]}, {t[13], t[14], t[16]}, {t[15], t[16], t[17]}};
+    const int axes = a.rotate ? 3 : 2, cols = axes + 1;
+    const int i = min(lane / cols, axes - 1), j = lane % cols;
+    bool good = solve;
+    double e = 0;
+    if (solve) {
       const F2 sn = f2_div(sum, n);
       const F2 inv_e = f2_div(f2(1.f), energy);
-      const F2 qi = f2_sub(t[6 + i], f2_mul(sn, gs[i]));
+      const F2 gsi = t[3 + i];
+      const F2 qi = f2_sub(t[6 + i], f2_mul(sn, gsi));
       if (j < axes) {
-        const F2 qj = f2_sub(t[6 + j], f2_mul(sn, gs[j]));
-        const F2 e = f2_sub(f2_sub(gg[i][j], f2_div(f2_mul(gs[i], gs[j]), n)), f2_mul(f2_mul(qi, qj), inv_e));
-        entry = f2_dbl(f2_mul(e, inv_e));
+        const F2 gsj = t[3 + j];
+        const F2 qj = f2_sub(t[6 + j], f2_mul(sn, gsj));
+        const int hi = max(i, j), lo = min(i, j);
+        const F2 gg = t[12 + hi * (hi + 1) / 2 + lo];
+        const F2 m = f2_sub(f2_sub(gg, f2_div(f2_mul(gsi, gsj), n)), f2_mul(f2_mul(qi, qj), inv_e));
+        e = f2_dbl(f2_mul(m, inv_e));
       } else {
-        entry = f2_dbl(f2_sub(f2_mul(f2(sign / sq), wg[i]), f2_mul(f2_mul(f2(score), qi), inv_e)));
+        e = f2_dbl(f2_sub(f2_mul(f2(sign / sq), t[9 + i]), f2_mul(f2_mul(f2(score), qi), inv_e)));
+      }
+      // Gauss-Jordan with partial pivoting
+      const int row = lane / cols;
+      for (int c = 0; c < axes; ++c) {
+        int pivot = c;
+        double pv = __shfl_sync(0xffffffffu, e, c * cols + c);
+        for (int r = c + 1; r < axes; ++r) {
+          const double v = __shfl_sync(0xffffffffu, e, r * cols + c);
+          if (fabs(v) > fabs(pv)) {
+            pv = v;
+            pivot = r;
+          }
+        }
+        if (fabs(pv) < 1e-14) {
+          good = false;
+          break;
+        }
+        const int from = row == c ? pivot * cols + j : row == pivot ? c * cols + j : lane;
+        e = __shfl_sync(0xffffffffu, e, from);
+        const double inv = 1.0 / pv;
+        if (row == c) e *= inv;
+        const double prow = __shfl_sync(0xffffffffu, e, c * cols + j);
+        const double g = __shfl_sync(0xffffffffu, e, min(row, axes - 1) * cols + c);
+        if (row != c) e -= g * prow;
       }
     }
-    double m[3][4];
-    for (int i = 0; i < 3; ++i)
-      for (int j = 0; j < 4; ++j) m[i][j] = 0;
-    for (int l = 0; l < axes * (axes + 1); ++l) {
-      const double v = __shfl_sync(0xffffffffu, entry, l);
-      m[l / (axes + 1)][l % (axes + 1)] = v;
-    }
+    const double d = __shfl_sync(0xffffffffu, e, lane < axes ? lane * cols + axes : 0);
+    const double mine = good && lane < axes ? d : 0.;
+    const bool finite = __all_sync(0xffffffffu, isfinite(mine));
+    if (lane < 3) f.gn_delta[lane] = mine;
     if (lane == 0) {
-      sh.ok = 0;
-      sh.gscore = gscore;
-      sh.delta[0] = sh.delta[1] = sh.delta[2] = 0;
-      if (solve) {
-        bool good = true;
-        for (int i = 0; i < axes && good; ++i) {
-          int pivot = i;
-          for (int j = i + 1; j < axes; ++j)
-            if (fabs(m[j][i]) > fabs(m[pivot][i])) pivot = j;
-          if (fabs(m[pivot][i]) < 1e-14) {
-            good = false;
-            break;
-          }
-          for (int k = i; k <= axes; ++k) {
-            const double tmp = m[i][k];
-            m[i][k] = m[pivot][k];
-            m[pivot][k] = tmp;
-          }
-          const double inv = 1.0 / m[i][i];
-          for (int k = i; k <= axes; ++k) m[i][k] *= inv;
-          for (int j = 0; j < axes; ++j)
-            if (j != i) {
-              const double f = m[j][i];
-              for (int k = i; k <= axes; ++k) m[j][k] -= f * m[i][k];
-            }
-        }
-        if (good) {
-          for (int i = 0; i < axes; ++i) sh.delta[i] = m[i][axes];
-          if (!rotate) sh.delta[2] = 0;
-          sh.ok = isfinite(sh.delta[0]) && isfinite(sh.delta[1]) && isfinite(sh.delta[2]);
-        }
-      }
+      f.ok = good && finite;
+      f.gscore = gscore;
     }
   }
   __syncthreads();
 }
 
-
-// Per-block fit state; scalar decisions are made by thread 0 and read by all
-// threads after a barrier.
-struct FitShared {
-  PoseShared ps;
-  Cand c, imp, best, seed;
-  double next_delta[3], delta[3], factor;
-  int cached, accepted, next_valid, flag;
-  float wbest[32];
-  int word[32];
-};
-
-__device__ __forceinline__ double local_row(const RefineArgs& a, double row) { return (row - a.crop_row - a.phase) / a.scale; }
-__device__ __forceinline__ double local_col(const RefineArgs& a, double col) { return (col - a.crop_col - a.phase) / a.scale; }
-
-__device__ void score_pose(const RefineArgs& a, FitShared& f, const Cand& p) {
-  continuous_pass(a.img, a.orig, local_row(a, p.row), local_col(a, p.col), p.angle, a.absolute, f.ps);
+__device__ __forceinline__ void local_pose(const RefineArgs& a, FitShared& f, const double* pose) {
+  set_local(f.lp, pose, a.crop_row, a.crop_col, a.phase, a.inv_scale);
 }
 
-__device__ __forceinline__ double step_factor(const double d[3], int rotate, double angle_step) {
-  double fct = fmin(1., fmin(.75 / fmax(1e-20, fabs(d[0])), .75 / fmax(1e-20, fabs(d[1]))));
-  if (rotate) fct = fmin(fct, angle_step / fmax(1e-20, fabs(d[2])));
-  return fct;
+// Score at the pose in f.lp, for every thread.
+__device__ __noinline__ double score_pass(const RefineArgs& a, FitShared& f) {
+  return continuous_pass(a.img, a.orig, f.lp, a.absolute, f.tot4);
 }
 
-// fit() of src/ncc_matching/matcher.cpp:903-982 for the candidate in f.c
-// (single-model query: no memo, no background guard).
-__device__ void fit_full(const RefineArgs& a, FitShared& f) {
-  if (!a.subpixel) return;
-  if (threadIdx.x == 0) f.cached = 0;
-  __syncthreads();
+// The step's factor from f.delta (warp 0): at most .75 rows and columns and
+// one angle step.
+__device__ __forceinline__ void step_factor(const RefineArgs& a, FitShared& f) {
+  const int lane = threadIdx.x;
+  double q = INFINITY;
+  if (lane < 2 || (lane == 2 && a.rotate)) q = (lane < 2 ? .75 : a.angle_step) / fmax(1e-20, fabs(f.delta[lane]));
+  const double q1 = __shfl_sync(0xffffffffu, q, 1), q2 = __shfl_sync(0xffffffffu, q, 2);
+  if (lane == 0) f.factor = fmin(fmin(1., fmin(q, q1)), q2);
+  __syncwarp();
+}
+
+// Trial pose number bt of the step (warp 0): half the last one's way, the
+// angle clamped; f.flag tells whether it lies in the domain, f.lp is its
+// local pose.  `unit`: level pixels per row and column of the step.
+__device__ __forceinline__ void trial_pose(const RefineArgs& a, FitShared& f, int bt, double unit) {
+  const int lane = threadIdx.x;
+  const double st = f.factor * (1. / double(1 << bt));  // exact
+  int pixel = 0;
+  if (lane < 3) {
+    const double s = lane < 2 ? dmul(unit, st) : st;
+    double v = dadd(f.pose[lane], dmul(s, f.delta[lane]));
+    if (lane == 2) v = fmin(fmax(v, a.angle_start), a.angle_end);
+    f.trial[lane] = v;
+    if (lane < 2) {
+      // domain_contains: the nearest pixel lies in the image (and the mask)
+      const double p = floor(v + .5);
+      pixel = p >= 0 && p < double(lane ? a.dom.w : a.dom.h) ? int(p) : -1;
+    }
+  }
+  const int r = __shfl_sync(0xffffffffu, pixel, 0), c = __shfl_sync(0xffffffffu, pixel, 1);
+  const bool in = r >= 0 && c >= 0 && (!a.dom.mask || a.dom.mask[size_t(r) * a.dom.w + size_t(c)] != 0);
+  if (lane == 0) f.flag = in;
+  __syncwarp();
+  if (in) local_pose(a, f, f.trial);
+}
+
+// fit() of src/ncc_matching/matcher.cpp:903-982 for the pose in f.pose with
+// score `score` (single-model query: no memo, no background guard); returns
+// the fitted pose's score.
+__device__ __noinline__ double fit_full(const RefineArgs& a, FitShared& f, double score) {
+  if (!a.subpixel) return score;
+  bool cached = false;  // f.next_delta is the step at f.pose
   for (int it = 0; it < 6; ++it) {
-    if (!f.cached) {
-      gn_pass(a.img, a.orig, local_row(a, f.c.row), local_col(a, f.c.col), f.c.angle, a.absolute, a.rotate, false, 0.,
-              f.ps);
-      if (!f.ps.ok) break;
-      if (threadIdx.x == 0)
-        for (int k = 0; k < 3; ++k) f.delta[k] = f.ps.delta[k];
-    } else if (threadIdx.x == 0) {
-      for (int k = 0; k < 3; ++k) f.delta[k] = f.next_delta[k];
+    if (!cached) {
+      if (threadIdx.x < 32) local_pose(a, f, f.pose);
+      __syncthreads();
+      gn_pass(a, f, false, 0.);
+      if (!f.ok) break;
     }
-    if (threadIdx.x == 0) {
-      f.cached = 0;
-      f.factor = step_factor(f.delta, a.rotate, a.angle_step);
-      f.accepted = 0;
-    }
-    __syncthreads();
-    for (int bt = 0; bt < 4; ++bt) {
-      if (threadIdx.x == 0) {
-        const double st = ldexp(f.factor, -bt);
-        Cand imp = f.c;
-        imp.row = dadd(imp.row, dmul(st, f.delta[0]));
-        imp.col = dadd(imp.col, dmul(st, f.delta[1]));
-        imp.angle = fmin(fmax(dadd(imp.angle, dmul(st, f.delta[2])), a.angle_start), a.angle_end);
-        f.imp = imp;
-        f.flag = domain_contains(a.dom, imp.row, imp.col);
-        f.next_valid = 0;
+    bool accepted = false, next_valid = false;
+    for (int bt = 0; bt < 4 && !accepted; ++bt) {
+      __syncthreads();  // f.lp, f.flag and the last pass's results have been read
+      if (threadIdx.x < 32) {
+        if (bt == 0) {
+          if (threadIdx.x < 3) f.delta[threadIdx.x] = cached ? f.next_delta[threadIdx.x] : f.gn_delta[threadIdx.x];
+          __syncwarp();
+          step_factor(a, f);
+        }
+        trial_pose(a, f, bt, 1.);
       }
       __syncthreads();
+      if (bt == 0) cached = false;
       if (!f.flag) continue;
+      double got;
       if (bt == 0 && it + 1 < 6) {
-        gn_pass(a.img, a.orig, local_row(a, f.imp.row), local_col(a, f.imp.col), f.imp.angle, a.absolute, a.rotate,
-                true, f.c.score, f.ps);
-        if (threadIdx.x == 0) {
-          f.imp.score = f.ps.gscore;
-          f.next_valid = f.ps.ok;
-          for (int k = 0; k < 3; ++k) f.next_delta[k] = f.ps.delta[k];
-        }
-        __syncthreads();
-        if (!isfinite(f.imp.score)) {
-          score_pose(a, f, f.imp);
-          if (threadIdx.x == 0) f.imp.score = f.ps.score;
-        }
+        gn_pass(a, f, true, score);
+        got = f.gscore;
+        next_valid = f.ok;
+        if (threadIdx.x < 3) f.next_delta[threadIdx.x] = f.gn_delta[threadIdx.x];
+        if (!isfinite(got)) got = score_pass(a, f);
       } else {
-        score_pose(a, f, f.imp);
-        if (threadIdx.x == 0) f.imp.score = f.ps.score;
+        next_valid = false;
+        got = score_pass(a, f);
       }
-      __syncthreads();
-      if (threadIdx.x == 0 && f.imp.score > f.c.score) {
-        f.c = f.imp;
-        f.accepted = 1;
-        f.cached = f.next_valid;
+      if (got > score) {
+        score = got;
+        accepted = true;
+        cached = next_valid;
+        if (threadIdx.x < 3) f.pose[threadIdx.x] = f.trial[threadIdx.x];
       }
-      __syncthreads();
-      if (f.accepted) break;
     }
-    if (threadIdx.x == 0)
-      f.flag = !f.accepted || (hypot(f.delta[0], f.delta[1]) < 1e-4 && fabs(f.delta[2]) < 1e-5);
+    if (!accepted) break;
+    if (threadIdx.x == 0) f.flag = hypot(f.delta[0], f.delta[1]) < 1e-4 && fabs(f.delta[2]) < 1e-5;
     __syncthreads();
     if (f.flag) break;
   }
   __syncthreads();
+  return score;
 }
 
 // refine_coarse_candidate of src/ncc_matching/matcher.cpp:853-877
-__device__ void fit_coarse(const RefineArgs& a, FitShared& f) {
-  if (!a.subpixel) return;
+__device__ __noinline__ double fit_coarse(const RefineArgs& a, FitShared& f, double score) {
+  if (!a.subpixel) return score;
   for (int it = 0; it < 6; ++it) {
-    gn_pass(a.img, a.orig, local_row(a, f.c.row), local_col(a, f.c.col), f.c.angle, a.absolute, a.rotate, false, 0.,
-            f.ps);
-    if (!f.ps.ok) break;
-    if (threadIdx.x == 0) {
-      for (int k = 0; k < 3; ++k) f.delta[k] = f.ps.delta[k];
-      f.factor = step_factor(f.delta, a.rotate, a.angle_step);
-      f.accepted = 0;
-    }
+    if (threadIdx.x < 32) local_pose(a, f, f.pose);
     __syncthreads();
-    for (int bt = 0; bt < 4; ++bt) {
-      if (threadIdx.x == 0) {
-        const double st = ldexp(f.factor, -bt);
-        Cand nx = f.c;
-        nx.row = dadd(nx.row, dmul(dmul(a.scale, st), f.delta[0]));
-        nx.col = dadd(nx.col, dmul(dmul(a.scale, st), f.delta[1]));
-        nx.angle = fmin(fmax(dadd(nx.angle, dmul(st, f.delta[2])), a.angle_start), a.angle_end);
-        f.imp = nx;
-        f.flag = domain_contains(a.dom, nx.row, nx.col);
+    gn_pass(a, f, false, 0.);
+    if (!f.ok) break;
+    bool accepted = false;
+    for (int bt = 0; bt < 4 && !accepted; ++bt) {
+      __syncthreads();
+      if (threadIdx.x < 32) {
+        if (bt == 0) {
+          if (threadIdx.x < 3) f.delta[threadIdx.x] = f.gn_delta[threadIdx.x];
+          __syncwarp();
+          step_factor(a, f);
+        }
+        trial_pose(a, f, bt, a.scale);
       }
       __syncthreads();
       if (!f.flag) continue;
-      score_pose(a, f, f.imp);
-      if (threadIdx.x == 0) {
-        f.imp.score = f.ps.score;
-        if (f.imp.score > f.c.score) {
-          f.c = f.imp;
-          f.accepted = 1;
-        }
+      const double got = score_pass(a, f);
+      if (got > score) {
+        score = got;
+        accepted = true;
+        if (threadIdx.x < 3) f.pose[threadIdx.x] = f.trial[threadIdx.x];
       }
-      __syncthreads();
-      if (f.accepted) break;
     }
-    if (!f.accepted) break;
+    if (!accepted) break;
+    __syncthreads();
   }
   __syncthreads();
+  return score;
 }
 
 // Discrete level-0 search around the seed (matcher.cpp:986-1059): one warp per
 // (patch, position), exact integer moments in the loop.  Leaves the first
-// strict maximum over (patch order, dr, dc) in f.best (score -inf if none).
-__device__ void recovery_search(const RefineArgs& a, FitShared& f) {
+// strict maximum over (patch order, dr, dc) in f.best and f.best_score (-inf if none).
+__device__ __noinline__ void recovery_search(const RefineArgs& a, FitShared& f) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  const Cand seed = f.seed;
+  const double seed_row = f.seed[0], seed_col = f.seed[1], seed_angle = f.seed[2];
   float best = -INFINITY;
   int border = INT32_MAX;
   int k = 0;
   for (int j = 0; j < a.nplist0; ++j) {
     const PatchDesc pd = a.view0.patches[a.plist0[j]];
-    if (fabs(pd.angle - seed.angle) > a.angle_step * 1.01) continue;
+    if (fabs(pd.angle - seed_angle) > a.angle_step * 1.01) continue;
     const PosRange rg = a.ranges0[j];
-    const int r0 = int(round(seed.row - a.crop_row - pd.orow)), c0 = int(round(seed.col - a.crop_col - pd.ocol));
+    const int r0 = int(round(seed_row - a.crop_row - pd.orow)), c0 = int(round(seed_col - a.crop_col - pd.ocol));
     for (int pos = warp; pos < 25; pos += nw) {
       const int r = r0 + pos / 5 - 2, c = c0 + pos % 5 - 2;
       if (r < rg.r0 || r >= rg.r1 || c < rg.c0 || c >= rg.c1) continue;
@@ -2326,25 +2382,26 @@ __device__ void recovery_search(const RefineArgs& a, FitShared& f) {
         bs = f.wbest[w];
         bo = f.word[w];
       }
-    Cand out = seed;
-    out.score = -INFINITY;
+    f.best[0] = seed_row;
+    f.best[1] = seed_col;
+    f.best[2] = seed_angle;
+    f.best_score = -INFINITY;
     if (bo != INT32_MAX && bs > -INFINITY) {
       int kk = 0;
       for (int j = 0; j < a.nplist0; ++j) {
         const PatchDesc pd = a.view0.patches[a.plist0[j]];
-        if (fabs(pd.angle - seed.angle) > a.angle_step * 1.01) continue;
+        if (fabs(pd.angle - seed_angle) > a.angle_step * 1.01) continue;
         if (kk == bo / 25) {
-          const int r0 = int(round(seed.row - a.crop_row - pd.orow)), c0 = int(round(seed.col - a.crop_col - pd.ocol));
-          out.row = double((long long)a.crop_row + r0 + (bo % 25) / 5 - 2) + pd.orow;
-          out.col = double((long long)a.crop_col + c0 + (bo % 25) % 5 - 2) + pd.ocol;
-          out.angle = pd.angle;
-          out.score = double(bs);
+          const int r0 = int(round(seed_row - a.crop_row - pd.orow)), c0 = int(round(seed_col - a.crop_col - pd.ocol));
+          f.best[0] = double((long long)a.crop_row + r0 + (bo % 25) / 5 - 2) + pd.orow;
+          f.best[1] = double((long long)a.crop_col + c0 + (bo % 25) % 5 - 2) + pd.ocol;
+          f.best[2] = pd.angle;
+          f.best_score = double(bs);
           break;
         }
         ++kk;
       }
     }
-    f.best = out;
   }
   __syncthreads();
 }
@@ -2352,55 +2409,59 @@ __device__ void recovery_search(const RefineArgs& a, FitShared& f) {
 constexpr int kRefineThreads = 512;
 
 // refine_candidate (src/ncc_matching/matcher.cpp:878-1061) for one queued
-// candidate per block.
-__global__ void __launch_bounds__(kRefineThreads) refine_kernel(RefineArgs a) {
+// candidate per block.  Bound by the latency of a chain of passes: gathers,
+// two reductions and FP64 algebra each.  Five 128^2 candidates (six
+// Gauss-Newton passes and four scores each): 0.385 -> 0.183 ms (19 shuffle trees
+// per warp and once more on warp 0, FP64 steps on one thread, one sample at a
+// time before).
+__global__ void __launch_bounds__(kRefineThreads) refine_kernel(const __grid_constant__ RefineArgs a) {
   __shared__ FitShared f;
   const int b = blockIdx.x;
   // a queued round after the end of the selection has nothing to refine
   if (a.batch_count < 0 && a.state->done) return;
   if (b >= (a.batch_count >= 0 ? a.batch_count : a.state->batch_count)) return;
-  const int i = a.batch[b];
-  if (threadIdx.x == 0) {
-    f.c = a.sorted[i];
-    f.seed = f.c;
-  }
+  const int i = a.batch[b], t = threadIdx.x;
+  double score = a.sorted[i].score;
+  if (t < 3) f.pose[t] = f.seed[t] = (&a.sorted[i].row)[t];
   __syncthreads();
   if (a.finest) {
-    fit_coarse(a, f);
+    score = fit_coarse(a, f, score);
   } else {
-    fit_full(a, f);
-    if (a.subpixel && a.top > 0 && f.c.score < a.min_score) {
+    score = fit_full(a, f, score);
+    if (a.subpixel && a.top > 0 && score < a.min_score) {
       recovery_search(a, f);
       // the search starts from the fitted candidate: only a strictly higher
       // discrete score moves it
-      if (threadIdx.x == 0) {
-        if (!(f.best.score > f.c.score)) f.best = f.c;
-        f.flag = f.best.row != f.c.row || f.best.col != f.c.col || f.best.angle != f.c.angle;
-      }
+      const bool move = f.best_score > score && (f.best[0] != f.pose[0] || f.best[1] != f.pose[1] || f.best[2] != f.pose[2]);
       __syncthreads();
-      if (f.flag) {
-        score_pose(a, f, f.best);
-        if (threadIdx.x == 0) {
-          f.best.score = f.ps.score;
-          f.seed = f.c;  // keep the fitted candidate
-          f.c = f.best;
+      if (move) {
+        const double fitted = score;
+        if (t < 3) {
+          f.seed[t] = f.pose[t];  // keep the fitted candidate
+          f.pose[t] = f.best[t];
         }
+        if (t < 32) local_pose(a, f, f.pose);
         __syncthreads();
-        fit_full(a, f);
-        if (threadIdx.x == 0 && !(f.c.score > f.seed.score)) f.c = f.seed;
-        __syncthreads();
+        score = score_pass(a, f);
+        score = fit_full(a, f, score);
+        if (!(score > fitted)) {
+          score = fitted;
+          if (t < 3) f.pose[t] = f.seed[t];
+          __syncthreads();
+        }
       }
     }
   }
-  if (threadIdx.x == 0) {
+  if (t == 0) {
     Refined r;
-    r.row = f.c.row;
-    r.col = f.c.col;
-    r.angle = f.c.angle;
-    r.score = f.c.score;
-    r.ok = (f.c.score >= a.min_score) && domain_contains(a.dom, f.c.row, f.c.col);
+    Cand c{};
+    r.row = c.row = f.pose[0];
+    r.col = c.col = f.pose[1];
+    r.angle = c.angle = f.pose[2];
+    r.score = score;
+    r.ok = (score >= a.min_score) && domain_contains(a.dom, r.row, r.col);
     r.pad = 0;
-    r.rect = make_rect(f.c, a.geom);
+    r.rect = make_rect(c, a.geom);
     a.refined[i] = r;
     __threadfence();
     a.refined_flag[i] = 2;
@@ -2548,8 +2609,8 @@ cudaError_t launch_refine4(const Refine4Args& a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_score(const ScoreArgs& a, int max_candidates, cudaStream_t s) {
-  score_kernel<<<max_candidates, 128, 0, s>>>(a);
+cudaError_t launch_score(const ScoreArgs& a, int max_candidates, cudaStream_t s, int sms) {
+  score_kernel<<<std::min(max_candidates, 48 * sms), 128, 0, s>>>(a);
   return cudaGetLastError();
 }
 

@@ -275,7 +275,7 @@ struct ScoreArgs {
   Cand* cand;
   const QueryState* state;
   int slot;
-  double crop_row, crop_col, scale, phase;
+  double crop_row, crop_col, phase, inv_scale;  // inv_scale: 1 / the level's scale (a power of two)
   int absolute;
 };
 
@@ -361,7 +361,7 @@ struct RefineArgs {
   const int32_t* batch;
   const QueryState* state;  // batch size in state->batch_count, unless
   int batch_count;          // ... this is >= 0 (a host-chosen batch)
-  double crop_row, crop_col, scale, phase;
+  double crop_row, crop_col, scale, phase, inv_scale;
   double angle_start, angle_end, angle_step, min_score;
   int rotate, subpixel, absolute, top, finest;
   double height, width;     // full image (domain test)
@@ -378,7 +378,7 @@ cudaError_t launch_coarse(const CoarseArgs& a, int max_bh, int max_bw, cudaStrea
 cudaError_t launch_nms(const NmsArgs& a, cudaStream_t s);
 cudaError_t launch_track(const TrackArgs& a, int max_candidates, cudaStream_t s, size_t smem_limit, int sms);
 cudaError_t launch_dedup(const DedupArgs& a, int max_candidates, cudaStream_t s);
-cudaError_t launch_score(const ScoreArgs& a, int max_candidates, cudaStream_t s);
+cudaError_t launch_score(const ScoreArgs& a, int max_candidates, cudaStream_t s, int sms);
 cudaError_t launch_adjoint(const AdjointArgs& a, cudaStream_t s);
 cudaError_t launch_refine4(const Refine4Args& a, cudaStream_t s);
 cudaError_t launch_sort(const SortArgs& a, int max_candidates, cudaStream_t s);
