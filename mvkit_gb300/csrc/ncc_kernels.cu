@@ -1681,8 +1681,8 @@ __global__ void __launch_bounds__(kSortSeg) sort_segments_kernel(SortArgs a) {
       finite = sort_emit(a, rank, i);
     }
   }
-  const unsigned m = __ballot_sync(0xffffffffu, finite);
-  if ((t & 31) == 0 && m) atomicAdd(&a.state->sorted_count, __popc(m));
+  const unsigned scored = __ballot_sync(0xffffffffu, finite);
+  if ((t & 31) == 0 && scored) atomicAdd(&a.state->sorted_count, __popc(scored));
 }
 
 // Merges groups of kSortFan sorted segments of `seg` entries (eight threads
