@@ -102,8 +102,7 @@ struct DevLevel {
   void append(const Raster& r) {
     PatchDesc d{};
     d.angle = r.angle;
-    d.orow = r.orow;
-    d.ocol = r.ocol;
+    d.set_origin(r.orow, r.ocol);
     d.rmin = r.rmin;
     d.rmax = r.rmax;
     d.cmin = r.cmin;
@@ -693,8 +692,8 @@ struct Workspace {
   DevBuf<float> tc_dots, coarse_dots;
   DevBuf<Cand> coarse_cand;
   DevBuf<int2> coarse_rc;
-  DevBuf<uint32_t> pairs;            // fp16 pairs of the finest level
-  int pairs_level = -1;              // the level `pairs` holds
+  DevBuf<uint32_t> quads;            // quads of the finest level
+  int quads_level = -1;              // the level `quads` holds
   DevBuf<uint8_t> dom_mask;          // search domain of the current find
   DevBuf<int32_t> dom_count, dom_row_run;
   DevBuf<int4> dom_runs;
@@ -1167,7 +1166,7 @@ struct Prepared {
   // copies of the refinement's images
   bool owned = false;
   DevBuf<float> lev0, fine;
-  DevBuf<uint32_t> pairs;
+  DevBuf<uint32_t> quads;
 };
 
 // One find on the current device.  stage >= 0 stops after that stage and
@@ -1554,13 +1553,13 @@ FindOutput run_find(mvg_ncc_model_s& m, const void* pixels, int type, int64_t W,
   }
   QueryState* st = ws.state.p;
   int32_t* err_flag = &st->error;
-  // an fp16-exact level 0 that is also the finest: its half2 pairs come with it
-  const bool pairs0 = finest == 0 && (type == 1 ? 65535.0 : 255.0) <= 2048.0;
-  if (pairs0) ws.pairs.reserve(size_t(lw[0]) * size_t(lh[0]));
+  // quads of the finest level (levels whose values fit 16 bits); level 0's come with it
+  const QuadShape quad = quad_shape(lw[finest], lh[finest], (type == 1 ? 65535.0 : 255.0) * std::ldexp(1., int(2 * finest)));
+  if (quad.bits) ws.quads.reserve(quad.words());
   {
     Span sp(kStPyramid, s, int(level_count));
     check(launch_pyramid0(dev_pixels, type, pitch_elems, int(crop_row), int(crop_col), lev[0], err_flag, s,
-                          pairs0 ? ws.pairs.p : nullptr),
+                          finest == 0 ? ws.quads.p : nullptr, quad.tiles),
           "pyramid0");
     for (size_t l = 1; l < level_count; ++l) check(launch_pyramid(lev[l - 1], lev[l], err_flag, s), "pyramid");
     // uint16: the tensor-core planes are centred on the data's own range
@@ -1863,16 +1862,15 @@ FindOutput run_find(mvg_ncc_model_s& m, const void* pixels, int type, int64_t W,
   geom.area = double(base.width) * double(base.height);
   const double fscale = std::ldexp(1., int(finest)), fphase = (fscale - 1) * .5;
   ImageView fine{lev[finest].v, lw[finest], lh[finest]};
-  if ((type == 1 ? 65535.0 : 255.0) * std::ldexp(1., int(2 * finest)) <= 2048.0) {
-    // fp16-exact level: half2 pairs halve the bilinear loads of the
-    // continuous score and the Gauss-Newton passes
-    if (!pairs0) {
-      ws.pairs.reserve(size_t(lw[finest]) * size_t(lh[finest]));
+  if (quad.bits) {
+    if (finest) {
       Span sp(kStScore, s, 1);
-      check(launch_pairs(lev[finest].v, lw[finest], lh[finest], ws.pairs.p, s), "pairs");
+      check(launch_quads(lev[finest].v, lw[finest], lh[finest], quad, ws.quads.p, s), "quads");
     }
-    fine.pairs = ws.pairs.p;
-    ws.pairs_level = int(finest);
+    fine.quads = ws.quads.p;
+    fine.bits = quad.bits;
+    fine.tiles = quad.tiles;
+    ws.quads_level = int(finest);
   }
   {
     ScoreArgs sa;
@@ -1996,11 +1994,11 @@ FindOutput run_find(mvg_ncc_model_s& m, const void* pixels, int type, int64_t W,
         check(cudaMemcpyAsync(prep->fine.p, lev[finest].v, nf * sizeof(float), cudaMemcpyDeviceToDevice, s), "fine");
         prep->ra.img.v = prep->fine.p;
       }
-      if (fine.pairs) {
-        prep->pairs.reserve(nf);
-        check(cudaMemcpyAsync(prep->pairs.p, fine.pairs, nf * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s),
-              "pairs");
-        prep->ra.img.pairs = prep->pairs.p;
+      if (fine.quads) {
+        prep->quads.reserve(quad.words());
+        check(cudaMemcpyAsync(prep->quads.p, fine.quads, quad.words() * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s),
+              "quads");
+        prep->ra.img.quads = prep->quads.p;
       }
     }
     check(cudaStreamSynchronize(s), "sync");
@@ -2205,7 +2203,7 @@ struct MultiRefiner {
       while (j < n && order[j].owner == order[i].owner) ++j;
       const Prepared& P = *preps[size_t(order[i].owner)];
       RefineArgs ra = P.ra;
-      if (!P.owned && ra.img.pairs && ws.pairs_level != P.finest) ra.img.pairs = nullptr;  // another model's level
+      if (!P.owned && ws.quads_level != P.finest) ra.img.bits = 0;  // another model's level
       ra.sorted = d_cand.p + i;
       ra.refined = d_ref.p + i;
       ra.refined_flag = d_flag.p + i;
@@ -2975,7 +2973,7 @@ int32_t mvg_ncc_score_gradient(const void* pixels, int32_t pixel_type, int64_t w
     ws.adj_grad.reserve(4 * n);
     check(cudaMemcpyAsync(ws.adj_poses.p, poses, 4 * n * sizeof(double), cudaMemcpyHostToDevice, s), "poses");
     AdjointArgs aa;
-    aa.img = ImageView{lev0.v, lev0.w, lev0.h, nullptr};
+    aa.img = ImageView{lev0.v, lev0.w, lev0.h};
     aa.orig = orig;
     aa.poses = ws.adj_poses.p;
     aa.n = int(count);
@@ -3034,7 +3032,7 @@ int32_t mvg_ncc_refine_similarity(const void* pixels, int32_t pixel_type, int64_
     check(cudaMemcpyAsync(ws.adj_poses.p, poses, 4 * n * sizeof(double), cudaMemcpyHostToDevice, s), "poses");
     const HostModel& hm = model_id->host;
     Refine4Args ra;
-    ra.img = ImageView{lev0.v, lev0.w, lev0.h, nullptr};
+    ra.img = ImageView{lev0.v, lev0.w, lev0.h};
     ra.orig = orig;
     ra.poses = ws.adj_poses.p;
     ra.score = ws.adj_score.p;

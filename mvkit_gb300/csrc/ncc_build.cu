@@ -407,8 +407,7 @@ void build_tables_device(const HostModel& m, const std::vector<int32_t>& lin_pit
         const ModelLevel& L = m.levels[size_t(level)];
         PatchDesc d{};
         d.angle = b.angle;
-        d.orow = b.unrotated ? L.orow : 0.;
-        d.ocol = b.unrotated ? L.ocol : 0.;
+        d.set_origin(b.unrotated ? L.orow : 0., b.unrotated ? L.ocol : 0.);
         d.rmin = bounds[size_t(q)].x;
         d.rmax = bounds[size_t(q)].y;
         d.cmin = bounds[size_t(q)].z;

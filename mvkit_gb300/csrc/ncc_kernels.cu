@@ -190,21 +190,50 @@ __device__ __forceinline__ bool better(float s, int o, float bs, int bo) {
 }
 
 // ------------------------------------------------------------------ pyramid
-// Level 0: the crop as float; with `pairs`, also the fp16 pairs (v[x],
-// v[x+1]) of pairs_kernel (last column repeated) for an fp16-exact level 0.
+// Word (8 bits) or word pair (16 bits) of a pixel's quad.
+template <int Bits> __device__ __forceinline__ uint32_t quad_at(int x, int y, int tiles) {
+  constexpr int W = Bits == 8 ? 8 : 4;  // tile width; tiles are 4 high
+  // ((y / 4) tiles + x / W) 4 W + (y mod 4) W + x mod W
+  return uint32_t((y & ~3) * ((tiles - 1) * W) + y * W + (x & ~(W - 1)) * 3 + x);
+}
+template <int Bits>
+__device__ __forceinline__ void quad_store(uint32_t* quads, uint32_t at, uint32_t a, uint32_t b, uint32_t c,
+                                           uint32_t d) {
+  if (Bits == 8)
+    quads[at] = a | b << 8 | c << 16 | d << 24;
+  else
+    reinterpret_cast<uint2*>(quads)[at] = make_uint2(a | b << 16, c | d << 16);
+}
+
+// Level 0: the crop as float; with `quads`, also the crop's quads.
 template <class T>
 __global__ void pyramid0_kernel(const T* __restrict__ src, int64_t pitch, int crop_row, int crop_col, LevelImage dst,
-                                uint32_t* __restrict__ pairs) {
+                                uint32_t* __restrict__ quads, int quad_tiles) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   const int r = blockIdx.y * blockDim.y + threadIdx.y;
   if (c >= dst.w || r >= dst.h) return;
   const T* row = src + (int64_t(crop_row) + r) * pitch + crop_col;
-  const float v = float(row[c]);
-  dst.v[size_t(r) * dst.w + c] = v;
-  if (pairs) {
-    const __half a = __float2half_rn(v), b = __float2half_rn(float(row[c + 1 < dst.w ? c + 1 : c]));
-    pairs[size_t(r) * dst.w + c] = uint32_t(__half_as_ushort(a)) | (uint32_t(__half_as_ushort(b)) << 16);
+  const uint32_t v = row[c];
+  dst.v[size_t(r) * dst.w + c] = float(v);
+  if (quads) {
+    const int c1 = c + 1 < dst.w ? c + 1 : c;
+    const T* next = r + 1 < dst.h ? row + pitch : row;
+    constexpr int Bits = 8 * sizeof(T);
+    quad_store<Bits>(quads, quad_at<Bits>(c, r, quad_tiles), v, row[c1], next[c], next[c1]);
   }
+}
+
+// Quads of a level held as float.
+template <int Bits>
+__global__ void quads_kernel(const float* __restrict__ v, int w, int h, int tiles, uint32_t* __restrict__ quads) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  const int r = blockIdx.y * blockDim.y + threadIdx.y;
+  if (c >= w || r >= h) return;
+  const int c1 = c + 1 < w ? c + 1 : c;
+  const float* row = v + size_t(r) * w;
+  const float* next = r + 1 < h ? row + w : row;
+  quad_store<Bits>(quads, quad_at<Bits>(c, r, tiles), uint32_t(row[c]), uint32_t(row[c1]), uint32_t(next[c]),
+                   uint32_t(next[c1]));
 }
 
 // level k+1 from level k: 2x2 sums with the reference's clamped neighbours
@@ -304,8 +333,8 @@ __global__ void __launch_bounds__(256) coarse_kernel(CoarseArgs a) {
   if (r >= h || c >= w) return;
   float score = -INFINITY;
   if (any && r >= rg.r0 && r < rg.r1 && c >= rg.c0 && c < rg.c1 &&
-      may_contain(a.dom, lattice_pose(a.crop_row, a.scale, r, pd.orow, a.phase),
-                  lattice_pose(a.crop_col, a.scale, c, pd.ocol, a.phase), a.scale)) {
+      (!a.dom.mask || may_contain(a.dom, lattice_pose(a.crop_row, a.scale, r, pd.orow, a.phase),
+                                  lattice_pose(a.crop_col, a.scale, c, pd.ocol, a.phase), a.scale))) {
     const int2* sw = a.view.sw + pd.sample_off;
     const float* base = tile + (threadIdx.y - pd.rmin) * TW + (threadIdx.x - pd.cmin);
     const int2 f0 = __ldg(sw);
@@ -371,8 +400,8 @@ __global__ void coarse_tc_score_kernel(CoarseTcArgs a) {
   float score = -INFINITY;
   const PatchDesc pd = a.view.patches[a.plist[j]];
   if (r >= rg.r0 && r < rg.r1 && c >= rg.c0 && c < rg.c1 &&
-      may_contain(a.dom, lattice_pose(a.crop_row, a.scale, r, pd.orow, a.phase),
-                  lattice_pose(a.crop_col, a.scale, c, pd.ocol, a.phase), a.scale)) {
+      (!a.dom.mask || may_contain(a.dom, lattice_pose(a.crop_row, a.scale, r, pd.orow, a.phase),
+                                  lattice_pose(a.crop_col, a.scale, c, pd.ocol, a.phase), a.scale))) {
     const int ci = (src * a.lat_r + r / 5) * a.lat_c + c / 5;
     const int pos = (r % 5) * 5 + c % 5, k = a.k_of[j];
     long long s1, s2;
@@ -450,11 +479,11 @@ __device__ __forceinline__ TrackCentre track_centre(const TrackArgs& a, const Ca
   }
   return t;
 }
-__device__ __forceinline__ int track_row(const TrackArgs& a, const TrackCentre& t, double orow) {
-  return a.exact32 ? int(roundf(__fsub_rn(t.x32r, float(orow)))) : int(round(dsub(t.xr, orow)));
+__device__ __forceinline__ int track_row(const TrackArgs& a, const TrackCentre& t, const PatchDesc& pd) {
+  return a.exact32 ? int(roundf(__fsub_rn(t.x32r, pd.orow32))) : int(round(dsub(t.xr, pd.orow)));
 }
-__device__ __forceinline__ int track_col(const TrackArgs& a, const TrackCentre& t, double ocol) {
-  return a.exact32 ? int(roundf(__fsub_rn(t.x32c, float(ocol)))) : int(round(dsub(t.xc, ocol)));
+__device__ __forceinline__ int track_col(const TrackArgs& a, const TrackCentre& t, const PatchDesc& pd) {
+  return a.exact32 ? int(roundf(__fsub_rn(t.x32c, pd.ocol32))) : int(round(dsub(t.xc, pd.ocol)));
 }
 
 __device__ __forceinline__ bool track_valid(const TrackArgs& a, const PatchDesc& pd, const PosRange& rg, int r, int c) {
@@ -689,7 +718,7 @@ __device__ void track_write(const TrackArgs& a, int i, const Cand& cd, float bes
     const int l = item % 25;
     const int32_t pi = a.plist[a.sel_idx[sel0 + item / 25]];
     const PatchDesc pd = a.view.patches[pi];
-    const int r = track_row(a, t, pd.orow) + l / 5 - 2, c = track_col(a, t, pd.ocol) + l % 5 - 2;
+    const int r = track_row(a, t, pd) + l / 5 - 2, c = track_col(a, t, pd) + l % 5 - 2;
     if (a.exact32) {
       out.row = double(lattice_pose32(float(a.crop_row), float(a.step), r, float(pd.orow), float(a.offset)));
       out.col = double(lattice_pose32(float(a.crop_col), float(a.step), c, float(pd.ocol), float(a.offset)));
@@ -730,7 +759,7 @@ __device__ __noinline__ void plain_dots(const TrackArgs& a, const Cand& cd, int 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const PatchDesc pd = a.view.patches[a.plist[a.sel_idx[a.sel_off[cd.patch] + k]]];
   const TrackCentre t = track_centre(a, cd);
-  const int row = track_row(a, t, pd.orow), col = track_col(a, t, pd.ocol);
+  const int row = track_row(a, t, pd), col = track_col(a, t, pd);
   const int cr = min(max(row, 0), a.lev.h - 1), cc = min(max(col, 0), a.lev.w - 1);
   const LevelWindow win{a.lev.v, a.lev.w, a.lev.h, row - 2, col - 2, a.lev.v[size_t(cr) * a.lev.w + cc]};
   part[warp][lane] = level_dots(win, a.view, pd, 0, 0, warp, blockDim.x >> 5);
@@ -764,7 +793,7 @@ __global__ void __launch_bounds__(32 * kTrackWarps, 8) track_warp_kernel(const _
     bool plain = false;
     if (lane < n) {
       const PatchDesc& pd = a.view.patches[a.plist[a.sel_idx[sel0 + lane]]];
-      plain = !tc || pd.orow != 0 || pd.ocol != 0;
+      plain = !tc || !pd.lattice;
     }
     const unsigned left = __ballot_sync(0xffffffffu, plain);
     int slot = 0;
@@ -776,7 +805,7 @@ __global__ void __launch_bounds__(32 * kTrackWarps, 8) track_warp_kernel(const _
     for (int k = warp; k < n; k += nwarps) {
       const int j = a.sel_idx[sel0 + k];
       const PatchDesc pd = a.view.patches[a.plist[j]];
-      const int r = track_row(a, t, pd.orow) + dr - 2, c = track_col(a, t, pd.ocol) + dc - 2;
+      const int r = track_row(a, t, pd) + dr - 2, c = track_col(a, t, pd) + dc - 2;
       if (lane >= 25 || !track_valid(a, pd, a.ranges[j], r, c)) continue;
       const float dot = left >> k & 1 ? s_dot[min(1, __popc(left & ((1u << k) - 1)))][lane]
                                       : track_tc_dot(a, pd, src, i, k, lane, r, c);
@@ -848,10 +877,10 @@ __global__ void __launch_bounds__(512) track_block_kernel(TrackArgs a) {
       int wr0 = INT32_MAX, wc0 = INT32_MAX, wr1 = INT32_MIN, wc1 = INT32_MIN;
       for (int k = lane; k < n; k += 32) {
         const PatchDesc pd = a.view.patches[a.plist[a.sel_idx[sel0 + k]]];
-        const int row = track_row(a, t, pd.orow), col = track_col(a, t, pd.ocol);
+        const int row = track_row(a, t, pd), col = track_col(a, t, pd);
         s_row[k] = row;
         s_col[k] = col;
-        const bool istc = tc && pd.orow == 0 && pd.ocol == 0 && k < kTcMaxP;
+        const bool istc = tc && pd.lattice && k < kTcMaxP;
         s_istc[k] = istc;
         if (!istc) {
           wr0 = min(wr0, row - 2 + pd.rmin);
@@ -1187,6 +1216,54 @@ __device__ __forceinline__ int split_floor(float v, float& frac) {
   return __float_as_int(t) - 0x4b400000;
 }
 
+// The four values of the bilinear cell at (x, y), which lies inside: loaded
+// from the quads (integers of 8 or 16 bits) or the level (Bits 0), and put
+// into floats when they are used (an integer under the exponent of 2^23).
+struct Cell {
+  float a, b, d, e;
+};
+__device__ __forceinline__ float quad_value(uint32_t q, uint32_t sel) {
+  return __uint_as_float(__byte_perm(q, 0x4b000000u, sel)) - 8388608.f;
+}
+template <int Bits> struct RawCell;
+template <> struct RawCell<8> {
+  uint32_t q = 0;
+  __device__ __forceinline__ void load(const ImageView& img, int x, int y) {
+    q = __ldg(img.quads + quad_at<8>(x, y, img.tiles));
+  }
+  __device__ __forceinline__ Cell cell() const {
+    return Cell{quad_value(q, 0x7440), quad_value(q, 0x7441), quad_value(q, 0x7442), quad_value(q, 0x7443)};
+  }
+};
+template <> struct RawCell<16> {
+  uint2 q = {0, 0};
+  __device__ __forceinline__ void load(const ImageView& img, int x, int y) {
+    q = __ldg(reinterpret_cast<const uint2*>(img.quads) + quad_at<16>(x, y, img.tiles));
+  }
+  __device__ __forceinline__ Cell cell() const {
+    return Cell{quad_value(q.x, 0x7410), quad_value(q.x, 0x7432), quad_value(q.y, 0x7410), quad_value(q.y, 0x7432)};
+  }
+};
+template <> struct RawCell<0> {
+  Cell c = {0.f, 0.f, 0.f, 0.f};
+  __device__ __forceinline__ void load(const ImageView& img, int x, int y) {
+    const float* v = img.v + (size_t(y) * img.w + x);
+    c = Cell{__ldg(v), __ldg(v + 1), __ldg(v + img.w), __ldg(v + img.w + 1)};
+  }
+  __device__ __forceinline__ Cell cell() const { return c; }
+};
+
+// The arithmetic of a sample with its fused operations spelled out, so that a
+// pass rounds alike whatever the code around it.
+// a b - c d and a b + c d: the first product is the fused one.
+__device__ __forceinline__ float fms2(float a, float b, float c, float d) { return __fmaf_rn(a, b, -__fmul_rn(c, d)); }
+__device__ __forceinline__ float fma2(float a, float b, float c, float d) { return __fmaf_rn(a, b, __fmul_rn(c, d)); }
+// (1 - f) a + f b
+__device__ __forceinline__ float mix(float f, float a, float b) { return fma2(__fsub_rn(1.f, f), a, f, b); }
+__device__ __forceinline__ float cell_value(const Cell& v, float fy, float fx) {
+  return mix(fy, mix(fx, v.a, v.b), mix(fx, v.d, v.e));
+}
+
 // FP32 score from pair totals of sum q, sum q^2, sum w q.
 __device__ __forceinline__ float pair_score(F2 sum, F2 sq, F2 dot, int n, int absolute, bool* ok) {
   const F2 var = f2_sub(sq, f2_div(f2_mul(sum, sum), f2(float(n))));
@@ -1197,8 +1274,48 @@ __device__ __forceinline__ float pair_score(F2 sum, F2 sq, F2 dot, int n, int ab
   return absolute ? fabsf(s) : s;
 }
 
+// Sums of the samples of a pose whose cells all lie inside: sum q, sum q^2,
+// sum w q.  Six samples per step, all loads issued before the arithmetic
+// (four 0.164 and 0.336 ms at 2048^2 and over a full circle, six 0.162 and
+// 0.324, eight with fewer blocks 0.163 and 0.367); each thread still adds its
+// samples in order s, s + blockDim.x, ...
+constexpr int kScoreUnroll = 6;
+template <int Bits>
+__device__ __forceinline__ void inside_sums(const ImageView& img, const OriginalView& orig, const LocalPose& L,
+                                            float offset, float (&acc)[4]) {
+  constexpr int U = kScoreUnroll;
+  const int stride = blockDim.x;
+  for (int s0 = threadIdx.x; s0 < orig.n; s0 += U * stride) {
+    float4 p[U];
+    float fy[U], fx[U];
+    RawCell<Bits> raw[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int s = s0 + u * stride;
+      p[u] = s < orig.n ? __ldg(orig.dcw + s) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const float y = __fadd_rn(L.fr, fms2(L.ca, p[u].x, L.sa, p[u].y));
+      const float x = __fadd_rn(L.fc, fma2(L.ca, p[u].y, L.sa, p[u].x));
+      const int iy = split_floor(y, fy[u]), ix = split_floor(x, fx[u]);
+      raw[u].load(img, L.C0 + ix, L.R0 + iy);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (s0 + u * stride >= orig.n) break;
+      const Cell v = raw[u].cell();
+      const float q = __fsub_rn(cell_value(v, fy[u], fx[u]), offset);
+      acc[0] += q;
+      acc[1] = fmaf(q, q, acc[1]);
+      acc[2] = fmaf(p[u].z, q, acc[2]);
+    }
+  }
+}
+
 // continuous() of src/ncc_matching/matcher.cpp:144-156 at a level-local pose;
 // every thread of the block calls it and gets the score.
+template <int Bits>
 __device__ __forceinline__ double continuous_pass(const ImageView& img, const OriginalView& orig, const LocalPose& lp,
                                                   int absolute, BlockTotals<4>& tot) {
   const LocalPose L = lp;
@@ -1216,51 +1333,7 @@ __device__ __forceinline__ double continuous_pass(const ImageView& img, const Or
   }
   float acc[4] = {0.f, 0.f, 0.f, 0.f};  // sum q, sum q^2, sum w q, out-of-image flag
   if (samples_inside(L, orig, hmin, hmax, wmin, wmax)) {
-    // every sample and its 2x2 neighbourhood is inside: no tests, 32-bit offsets
-    const float* base = img.v + (size_t(L.R0) * img.w + L.C0);
-    const uint32_t* pbase = img.pairs ? img.pairs + (size_t(L.R0) * img.w + L.C0) : nullptr;
-    const int w = img.w;
-    // four samples per step, all loads issued before the arithmetic; each
-    // thread still adds its samples in order s, s + blockDim.x, ...
-    constexpr int U = 4;
-    const int stride = blockDim.x;
-    for (int s0 = threadIdx.x; s0 < orig.n; s0 += U * stride) {
-      float4 p[U];
-      float fy[U], fx[U], va[U], vb[U], vd[U], ve[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int s = s0 + u * stride;
-        p[u] = s < orig.n ? __ldg(orig.dcw + s) : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const float y = L.fr + (L.ca * p[u].x - L.sa * p[u].y), x = L.fc + (L.sa * p[u].x + L.ca * p[u].y);
-        const int iy = split_floor(y, fy[u]), ix = split_floor(x, fx[u]);
-        if (pbase) {
-          const uint32_t* pp = pbase + (iy * w + ix);
-          const uint32_t aq = __ldg(pp), bq = __ldg(pp + w);
-          va[u] = __half2float(__ushort_as_half(aq & 0xffff));
-          vb[u] = __half2float(__ushort_as_half(aq >> 16));
-          vd[u] = __half2float(__ushort_as_half(bq & 0xffff));
-          ve[u] = __half2float(__ushort_as_half(bq >> 16));
-        } else {
-          const float* v = base + (iy * w + ix);
-          va[u] = __ldg(v);
-          vb[u] = __ldg(v + 1);
-          vd[u] = __ldg(v + w);
-          ve[u] = __ldg(v + w + 1);
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        if (s0 + u * stride >= orig.n) break;
-        const float q = (1 - fy[u]) * ((1 - fx[u]) * va[u] + fx[u] * vb[u]) +
-                        fy[u] * ((1 - fx[u]) * vd[u] + fx[u] * ve[u]) - offset;
-        acc[0] += q;
-        acc[1] = fmaf(q, q, acc[1]);
-        acc[2] = fmaf(p[u].z, q, acc[2]);
-      }
-    }
+    inside_sums<Bits>(img, orig, L, offset, acc);
   } else
   for (int s = threadIdx.x; s < orig.n; s += blockDim.x) {
     const float dr = __ldg(orig.dr + s), dc = __ldg(orig.dc + s), w = __ldg(orig.w + s);
@@ -1283,7 +1356,12 @@ __device__ __forceinline__ double continuous_pass(const ImageView& img, const Or
   return ok ? double(sc) : -INFINITY;
 }
 
-__global__ void __launch_bounds__(128, 12) score_kernel(ScoreArgs a) {
+// Full-resolution score of every candidate.  Bound by the latency of the
+// gathers and the instructions around them (some 55 per 32 samples, one
+// gather).  Quads against row-major values: 4096^2 uint16 with a 256^2
+// template 3.17 -> 1.35 ms, 1024x1280 full circle with 48^2 0.52 -> 0.32 ms
+// (0.40 of it the folded reduction), 2048^2 uint8 0.172 -> 0.162 ms.
+template <int Bits> __global__ void __launch_bounds__(128, 12) score_kernel(ScoreArgs a) {
   __shared__ BlockTotals<4> tot;
   __shared__ LocalPose lp;
   const int live = live_count(a.state, a.slot);
@@ -1294,7 +1372,7 @@ __global__ void __launch_bounds__(128, 12) score_kernel(ScoreArgs a) {
     if (!isfinite(c.score)) continue;
     if (threadIdx.x < 32) set_local(lp, &c.row, a.crop_row, a.crop_col, a.phase, a.inv_scale);
     __syncthreads();
-    const double score = continuous_pass(a.img, a.orig, lp, a.absolute, tot);
+    const double score = continuous_pass<Bits>(a.img, a.orig, lp, a.absolute, tot);
     if (threadIdx.x == 0) a.cand[i].score = score;
   }
 }
@@ -1600,15 +1678,6 @@ __global__ void __launch_bounds__(kRefine4Threads) refine4_kernel(Refine4Args a)
 }
 
 // --------------------------------------------------------------------- sort
-// fp16 pairs (v[x], v[x+1]) of an fp16-exact level (last column repeats).
-__global__ void pairs_kernel(const float* __restrict__ v, int w, int h, uint32_t* __restrict__ out) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (long long)w * h) return;
-  const int x = int(i % w);
-  const __half a = __float2half_rn(v[i]), b = __float2half_rn(v[x + 1 < w ? i + 1 : i]);
-  out[i] = uint32_t(__half_as_ushort(a)) | (uint32_t(__half_as_ushort(b)) << 16);
-}
-
 // 64-bit keys ordering scores descending (order-preserving bit transform).
 __device__ __forceinline__ unsigned long long desc_key(double s) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(s);
@@ -2021,6 +2090,7 @@ struct FitShared {
 // f.gn_delta hold the result, for every thread.  Kept out of line: its code
 // runs once per pass and is called from several places, and copies of it
 // would miss the instruction cache.
+template <int Bits>
 __device__ __noinline__ void gn_pass(const RefineArgs& a, FitShared& f, bool use_minimum, double minimum) {
   const ImageView& img = a.img;
   const OriginalView& orig = a.orig;
@@ -2042,15 +2112,14 @@ __device__ __noinline__ void gn_pass(const RefineArgs& a, FitShared& f, bool use
 #pragma unroll
   for (int k = 0; k < 19; ++k) acc[k] = 0.f;
   const bool inside = samples_inside(L, orig, hmin, hmax, wmin, wmax);
-  const float* base = img.v + (size_t(L.R0) * img.w + L.C0);
-  const uint32_t* pbase = inside && img.pairs ? img.pairs + (size_t(L.R0) * img.w + L.C0) : nullptr;
-  const int w = img.w, stride = blockDim.x;
+  const int stride = blockDim.x;
   // four samples per step, all loads issued before the arithmetic; each
   // thread still adds its samples in order s, s + blockDim.x, ...
   constexpr int U = 4;
   for (int s0 = threadIdx.x; s0 < orig.n; s0 += U * stride) {
     float4 p[U];
-    float fy[U], fx[U], va[U], vb[U], vd[U], ve[U];
+    float fy[U], fx[U];
+    RawCell<Bits> raw[U];
     bool in[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -2060,38 +2129,24 @@ __device__ __noinline__ void gn_pass(const RefineArgs& a, FitShared& f, bool use
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const float y = L.fr + (L.ca * p[u].x - L.sa * p[u].y), x = L.fc + (L.sa * p[u].x + L.ca * p[u].y);
+      const float y = __fadd_rn(L.fr, fms2(L.ca, p[u].x, L.sa, p[u].y));
+      const float x = __fadd_rn(L.fc, fma2(L.sa, p[u].x, L.ca, p[u].y));
       if (!inside && in[u] && !(y >= hmin && x >= wmin && y < hmax && x < wmax)) {
         acc[18] = 1.f;
         in[u] = false;
       }
       const int iy = split_floor(y, fy[u]), ix = split_floor(x, fx[u]);
-      va[u] = vb[u] = vd[u] = ve[u] = 0.f;
-      if (!in[u]) continue;
-      if (pbase) {
-        const uint32_t* pp = pbase + (iy * w + ix);
-        const uint32_t aq = __ldg(pp), bq = __ldg(pp + w);
-        va[u] = __half2float(__ushort_as_half(aq & 0xffff));
-        vb[u] = __half2float(__ushort_as_half(aq >> 16));
-        vd[u] = __half2float(__ushort_as_half(bq & 0xffff));
-        ve[u] = __half2float(__ushort_as_half(bq >> 16));
-      } else {
-        const float* v = base + (iy * w + ix);
-        va[u] = __ldg(v);
-        vb[u] = __ldg(v + 1);
-        vd[u] = __ldg(v + w);
-        ve[u] = __ldg(v + w + 1);
-      }
+      if (in[u]) raw[u].load(img, L.C0 + ix, L.R0 + iy);
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       if (!in[u]) continue;
+      const Cell v = raw[u].cell();
       const float dr = p[u].x, dc = p[u].y, wt = p[u].z;
-      const float q = (1 - fy[u]) * ((1 - fx[u]) * va[u] + fx[u] * vb[u]) +
-                      fy[u] * ((1 - fx[u]) * vd[u] + fx[u] * ve[u]) - offset;
-      const float gy = (1 - fx[u]) * (vd[u] - va[u]) + fx[u] * (ve[u] - vb[u]),
-                  gx = (1 - fy[u]) * (vb[u] - va[u]) + fy[u] * (ve[u] - vd[u]);
-      const float g2 = gy * (-L.sa * dr - L.ca * dc) + gx * (L.ca * dr - L.sa * dc);
+      const float q = __fsub_rn(cell_value(v, fy[u], fx[u]), offset);
+      const float gy = mix(fx[u], __fsub_rn(v.d, v.a), __fsub_rn(v.e, v.b));
+      const float gx = mix(fy[u], __fsub_rn(v.b, v.a), __fsub_rn(v.e, v.d));
+      const float g2 = fma2(gy, fms2(-L.sa, dr, L.ca, dc), gx, fms2(L.ca, dr, L.sa, dc));
       acc[0] += q;
       acc[1] = fmaf(q, q, acc[1]);
       acc[2] = fmaf(wt, q, acc[2]);
@@ -2190,8 +2245,8 @@ __device__ __forceinline__ void local_pose(const RefineArgs& a, FitShared& f, co
 }
 
 // Score at the pose in f.lp, for every thread.
-__device__ __noinline__ double score_pass(const RefineArgs& a, FitShared& f) {
-  return continuous_pass(a.img, a.orig, f.lp, a.absolute, f.tot4);
+template <int Bits> __device__ __noinline__ double score_pass(const RefineArgs& a, FitShared& f) {
+  return continuous_pass<Bits>(a.img, a.orig, f.lp, a.absolute, f.tot4);
 }
 
 // The step's factor from f.delta (warp 0): at most .75 rows and columns and
@@ -2233,14 +2288,14 @@ __device__ __forceinline__ void trial_pose(const RefineArgs& a, FitShared& f, in
 // fit() of src/ncc_matching/matcher.cpp:903-982 for the pose in f.pose with
 // score `score` (single-model query: no memo, no background guard); returns
 // the fitted pose's score.
-__device__ __noinline__ double fit_full(const RefineArgs& a, FitShared& f, double score) {
+template <int Bits> __device__ __noinline__ double fit_full(const RefineArgs& a, FitShared& f, double score) {
   if (!a.subpixel) return score;
   bool cached = false;  // f.next_delta is the step at f.pose
   for (int it = 0; it < 6; ++it) {
     if (!cached) {
       if (threadIdx.x < 32) local_pose(a, f, f.pose);
       __syncthreads();
-      gn_pass(a, f, false, 0.);
+      gn_pass<Bits>(a, f, false, 0.);
       if (!f.ok) break;
     }
     bool accepted = false, next_valid = false;
@@ -2259,14 +2314,14 @@ __device__ __noinline__ double fit_full(const RefineArgs& a, FitShared& f, doubl
       if (!f.flag) continue;
       double got;
       if (bt == 0 && it + 1 < 6) {
-        gn_pass(a, f, true, score);
+        gn_pass<Bits>(a, f, true, score);
         got = f.gscore;
         next_valid = f.ok;
         if (threadIdx.x < 3) f.next_delta[threadIdx.x] = f.gn_delta[threadIdx.x];
-        if (!isfinite(got)) got = score_pass(a, f);
+        if (!isfinite(got)) got = score_pass<Bits>(a, f);
       } else {
         next_valid = false;
-        got = score_pass(a, f);
+        got = score_pass<Bits>(a, f);
       }
       if (got > score) {
         score = got;
@@ -2285,12 +2340,12 @@ __device__ __noinline__ double fit_full(const RefineArgs& a, FitShared& f, doubl
 }
 
 // refine_coarse_candidate of src/ncc_matching/matcher.cpp:853-877
-__device__ __noinline__ double fit_coarse(const RefineArgs& a, FitShared& f, double score) {
+template <int Bits> __device__ __noinline__ double fit_coarse(const RefineArgs& a, FitShared& f, double score) {
   if (!a.subpixel) return score;
   for (int it = 0; it < 6; ++it) {
     if (threadIdx.x < 32) local_pose(a, f, f.pose);
     __syncthreads();
-    gn_pass(a, f, false, 0.);
+    gn_pass<Bits>(a, f, false, 0.);
     if (!f.ok) break;
     bool accepted = false;
     for (int bt = 0; bt < 4 && !accepted; ++bt) {
@@ -2305,7 +2360,7 @@ __device__ __noinline__ double fit_coarse(const RefineArgs& a, FitShared& f, dou
       }
       __syncthreads();
       if (!f.flag) continue;
-      const double got = score_pass(a, f);
+      const double got = score_pass<Bits>(a, f);
       if (got > score) {
         score = got;
         accepted = true;
@@ -2411,9 +2466,10 @@ constexpr int kRefineThreads = 512;
 // refine_candidate (src/ncc_matching/matcher.cpp:878-1061) for one queued
 // candidate per block.  Bound by the latency of a chain of passes: gathers,
 // two reductions and FP64 algebra each.  Five 128^2 candidates (six
-// Gauss-Newton passes and four scores each): 0.385 -> 0.183 ms (19 shuffle trees
+// Gauss-Newton passes and four scores each): 0.385 -> 0.177 ms (19 shuffle trees
 // per warp and once more on warp 0, FP64 steps on one thread, one sample at a
 // time before).
+template <int Bits>
 __global__ void __launch_bounds__(kRefineThreads) refine_kernel(const __grid_constant__ RefineArgs a) {
   __shared__ FitShared f;
   const int b = blockIdx.x;
@@ -2425,9 +2481,9 @@ __global__ void __launch_bounds__(kRefineThreads) refine_kernel(const __grid_con
   if (t < 3) f.pose[t] = f.seed[t] = (&a.sorted[i].row)[t];
   __syncthreads();
   if (a.finest) {
-    score = fit_coarse(a, f, score);
+    score = fit_coarse<Bits>(a, f, score);
   } else {
-    score = fit_full(a, f, score);
+    score = fit_full<Bits>(a, f, score);
     if (a.subpixel && a.top > 0 && score < a.min_score) {
       recovery_search(a, f);
       // the search starts from the fitted candidate: only a strictly higher
@@ -2442,8 +2498,8 @@ __global__ void __launch_bounds__(kRefineThreads) refine_kernel(const __grid_con
         }
         if (t < 32) local_pose(a, f, f.pose);
         __syncthreads();
-        score = score_pass(a, f);
-        score = fit_full(a, f, score);
+        score = score_pass<Bits>(a, f);
+        score = fit_full<Bits>(a, f, score);
         if (!(score > fitted)) {
           score = fitted;
           if (t < 3) f.pose[t] = f.seed[t];
@@ -2520,15 +2576,15 @@ cudaError_t reserve_dynamic_smem(const void* kernel, size_t bytes) {
 }
 
 cudaError_t launch_pyramid0(const void* src, int type, int64_t pitch_elems, int crop_row, int crop_col, LevelImage dst,
-                            int32_t* error_flag, cudaStream_t s, uint32_t* pairs) {
+                            int32_t* error_flag, cudaStream_t s, uint32_t* quads, int quad_tiles) {
   (void)error_flag;
   const dim3 block(32, 8), grid((dst.w + 31) / 32, (dst.h + 7) / 8);
   if (type == 1)
     pyramid0_kernel<uint16_t><<<grid, block, 0, s>>>(static_cast<const uint16_t*>(src), pitch_elems, crop_row, crop_col,
-                                                     dst, pairs);
+                                                     dst, quads, quad_tiles);
   else
     pyramid0_kernel<uint8_t><<<grid, block, 0, s>>>(static_cast<const uint8_t*>(src), pitch_elems, crop_row, crop_col,
-                                                    dst, pairs);
+                                                    dst, quads, quad_tiles);
   return cudaGetLastError();
 }
 
@@ -2610,7 +2666,12 @@ cudaError_t launch_refine4(const Refine4Args& a, cudaStream_t s) {
 }
 
 cudaError_t launch_score(const ScoreArgs& a, int max_candidates, cudaStream_t s, int sms) {
-  score_kernel<<<std::min(max_candidates, 48 * sms), 128, 0, s>>>(a);
+  const int grid = std::min(max_candidates, 48 * sms);
+  switch (a.img.bits) {
+    case 8: score_kernel<8><<<grid, 128, 0, s>>>(a); break;
+    case 16: score_kernel<16><<<grid, 128, 0, s>>>(a); break;
+    default: score_kernel<0><<<grid, 128, 0, s>>>(a); break;
+  }
   return cudaGetLastError();
 }
 
@@ -2628,9 +2689,14 @@ cudaError_t launch_coarse_tc_score(const CoarseTcArgs& a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_pairs(const float* v, int w, int h, uint32_t* pairs, cudaStream_t s) {
-  const long long n = (long long)w * h;
-  pairs_kernel<<<unsigned((n + 255) / 256), 256, 0, s>>>(v, w, h, pairs);
+cudaError_t launch_quads(const float* v, int w, int h, const QuadShape& shape, uint32_t* quads, cudaStream_t s) {
+  const dim3 block(32, 8), grid((w + 31) / 32, (h + 7) / 8);
+  if (shape.bits == 8)
+    quads_kernel<8><<<grid, block, 0, s>>>(v, w, h, shape.tiles, quads);
+  else if (shape.bits == 16)
+    quads_kernel<16><<<grid, block, 0, s>>>(v, w, h, shape.tiles, quads);
+  else
+    return cudaErrorInvalidValue;
   return cudaGetLastError();
 }
 
@@ -2657,7 +2723,11 @@ cudaError_t launch_select(const SelectArgs& a, cudaStream_t s) {
 }
 
 cudaError_t launch_refine(const RefineArgs& a, int batch_limit, cudaStream_t s) {
-  refine_kernel<<<batch_limit, kRefineThreads, 0, s>>>(a);
+  switch (a.img.bits) {
+    case 8: refine_kernel<8><<<batch_limit, kRefineThreads, 0, s>>>(a); break;
+    case 16: refine_kernel<16><<<batch_limit, kRefineThreads, 0, s>>>(a); break;
+    default: refine_kernel<0><<<batch_limit, kRefineThreads, 0, s>>>(a); break;
+  }
   return cudaGetLastError();
 }
 

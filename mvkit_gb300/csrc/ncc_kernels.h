@@ -244,9 +244,22 @@ cudaError_t launch_coarse_tc_score(const CoarseTcArgs& a, cudaStream_t s);
 // (h + 1) x (w + 1) prefix counts of a domain mask (DomainView::count)
 cudaError_t launch_domain_count(const uint8_t* mask, int w, int h, int32_t* count, cudaStream_t s);
 
-// half2 pairs (v[x], v[min(x + 1, w - 1)]) of a level whose values are exact
-// in fp16, w x h entries.
-cudaError_t launch_pairs(const float* v, int w, int h, uint32_t* pairs, cudaStream_t s);
+// Quads of a level whose values fit 8 or 16 bits: per pixel the four values
+// of its bilinear cell, (x, y), (x + 1, y), (x, y + 1), (x + 1, y + 1) from
+// the low end up (the last row and column repeat), in 4 or 8 bytes.  The
+// pixels of 8 x 4 (8 bits) or 4 x 4 (16 bits) tiles share a 128-byte line,
+// row by row, tile by tile: the samples of a rotated row touch a line per
+// several pixels in either direction, where a row-major image gives a line
+// per image row.
+struct QuadShape {
+  int bits, tiles, tile_rows;
+  size_t words() const { return size_t(tiles) * size_t(tile_rows) * 32; }
+};
+inline QuadShape quad_shape(int w, int h, double max_value) {
+  const int bits = max_value <= 255 ? 8 : max_value <= 65535 ? 16 : 0;
+  return QuadShape{bits, bits == 8 ? (w + 7) / 8 : (w + 3) / 4, (h + 3) / 4};
+}
+cudaError_t launch_quads(const float* v, int w, int h, const QuadShape& shape, uint32_t* quads, cudaStream_t s);
 
 struct DedupArgs {
   const Cand* in;
@@ -264,9 +277,10 @@ struct DedupArgs {
 struct ImageView {
   const float* v;           // finest level (float of pixel sums)
   int w, h;
-  // optional: per pixel the fp16 pair (v[x], v[x+1]) as half2 bits, for
-  // levels whose values are exact in fp16 (two loads per bilinear tap)
-  const uint32_t* pairs = nullptr;
+  // optional: quads of the level (below): one load per bilinear tap
+  const uint32_t* quads = nullptr;
+  int bits = 0;             // 8 or 16 bits per value (0: no quads)
+  int tiles = 0;            // tiles per row
 };
 
 struct ScoreArgs {
@@ -369,9 +383,9 @@ struct RefineArgs {
   DomainView dom;
 };
 
-// Level 0 (float crop); with `pairs`, also its fp16 pairs (launch_pairs' output)
+// Level 0 (float crop); with `quads`, also its quads (launch_quads' output)
 cudaError_t launch_pyramid0(const void* src, int type, int64_t pitch_elems, int crop_row, int crop_col, LevelImage dst,
-                            int32_t* error_flag, cudaStream_t s, uint32_t* pairs = nullptr);
+                            int32_t* error_flag, cudaStream_t s, uint32_t* quads = nullptr, int quad_tiles = 0);
 cudaError_t launch_pyramid(const LevelImage& src, LevelImage dst, int32_t* error_flag, cudaStream_t s);
 cudaError_t launch_prefix(const LevelImage& lev, cudaStream_t s);
 cudaError_t launch_coarse(const CoarseArgs& a, int max_bh, int max_bw, cudaStream_t s, size_t smem_limit);

@@ -37,7 +37,15 @@ struct PatchDesc {
   int32_t nruns;                // contiguous row spans
   int32_t run_off;
   float wsum;                   // sum of the float sample weights
-  int32_t pad_;
+  int32_t lattice;              // 1: the origin is on the lattice (orow = ocol = 0)
+  float orow32, ocol32;         // the origin in FP32
+  void set_origin(double row, double col) {
+    orow = row;
+    ocol = col;
+    lattice = row == 0 && col == 0;
+    orow32 = float(row);
+    ocol32 = float(col);
+  }
 };
 
 // Device view of one model level (its patches and their samples).
