@@ -2960,20 +2960,13 @@ int32_t mvg_ncc_score_gradient(const void* pixels, int32_t pixel_type, int64_t w
       check(cudaMemcpyAsync(ws.image.p, pixels, bytes, cudaMemcpyHostToDevice, s), "image upload");
       dev = ws.image.p;
     }
-    init_state(ws, s, kMaxCandidates);
-    LevelImage lev0{};
-    ws.lev_v[0].reserve(size_t(width) * size_t(height));
-    lev0.v = ws.lev_v[0].p;
-    lev0.w = int(width);
-    lev0.h = int(height);
-    check(launch_pyramid0(dev, pixel_type, row_stride / bpp, 0, 0, lev0, &ws.state.p->error, s), "pyramid0");
     const size_t n = size_t(count);
     ws.adj_poses.reserve(4 * n);
     ws.adj_score.reserve(n);
     ws.adj_grad.reserve(4 * n);
     check(cudaMemcpyAsync(ws.adj_poses.p, poses, 4 * n * sizeof(double), cudaMemcpyHostToDevice, s), "poses");
     AdjointArgs aa;
-    aa.img = ImageView{lev0.v, lev0.w, lev0.h};
+    aa.img = PixelView{dev, row_stride / bpp, int(width), int(height), pixel_type};
     aa.orig = orig;
     aa.poses = ws.adj_poses.p;
     aa.n = int(count);
@@ -3019,20 +3012,13 @@ int32_t mvg_ncc_refine_similarity(const void* pixels, int32_t pixel_type, int64_
       check(cudaMemcpyAsync(ws.image.p, pixels, bytes, cudaMemcpyHostToDevice, s), "image upload");
       dev = ws.image.p;
     }
-    init_state(ws, s, kMaxCandidates);
-    LevelImage lev0{};
-    ws.lev_v[0].reserve(size_t(width) * size_t(height));
-    lev0.v = ws.lev_v[0].p;
-    lev0.w = int(width);
-    lev0.h = int(height);
-    check(launch_pyramid0(dev, pixel_type, row_stride / bpp, 0, 0, lev0, &ws.state.p->error, s), "pyramid0");
     const size_t n = size_t(count);
     ws.adj_poses.reserve(4 * n);
     ws.adj_score.reserve(n);
     check(cudaMemcpyAsync(ws.adj_poses.p, poses, 4 * n * sizeof(double), cudaMemcpyHostToDevice, s), "poses");
     const HostModel& hm = model_id->host;
     Refine4Args ra;
-    ra.img = ImageView{lev0.v, lev0.w, lev0.h};
+    ra.img = PixelView{dev, row_stride / bpp, int(width), int(height), pixel_type};
     ra.orig = orig;
     ra.poses = ws.adj_poses.p;
     ra.score = ws.adj_score.p;

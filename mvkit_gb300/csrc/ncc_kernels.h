@@ -283,6 +283,14 @@ struct ImageView {
   int tiles = 0;            // tiles per row
 };
 
+// The search image as the caller holds it.
+struct PixelView {
+  const void* v;
+  int64_t pitch;            // in pixels
+  int w, h;
+  int type;                 // 0: uint8, 1: uint16
+};
+
 struct ScoreArgs {
   ImageView img;
   OriginalView orig;
@@ -297,7 +305,7 @@ struct ScoreArgs {
 // column, angle, scale; pixel-centre image coordinates, the model origin at
 // (row, column)) and its gradient in the four parameters.  One block per pose.
 struct AdjointArgs {
-  ImageView img;            // level 0: the search image as float
+  PixelView img;            // the search image
   OriginalView orig;
   const double* poses;      // n x 4
   int n;
@@ -310,7 +318,7 @@ struct AdjointArgs {
 // on the NCC above: the reference's refinement step (3 parameters,
 // src/ncc_matching/matcher.cpp:170-240, 903-982) with scale as a fourth.
 struct Refine4Args {
-  ImageView img;
+  PixelView img;
   OriginalView orig;
   double* poses;            // n x 4, refined in place
   double* score;            // n: score at the final pose (-inf if unscorable)
