@@ -3028,7 +3028,7 @@ int32_t mvg_ncc_refine_similarity(const void* pixels, int32_t pixel_type, int64_
     ra.max_shift = .75;  // as the reference's step limit (matcher.cpp:931)
     ra.max_angle = hm.params.angle_extent > 0 ? hm.params.angle_step : .01;
     ra.max_scale = .01;
-    check(launch_refine4(ra, s), "refine4");
+    check(launch_refine4(ra, s, ws.sm_count), "refine4");
     check(cudaMemcpyAsync(poses, ws.adj_poses.p, 4 * n * sizeof(double), cudaMemcpyDeviceToHost, s), "poses");
     check(cudaMemcpyAsync(score, ws.adj_score.p, n * sizeof(double), cudaMemcpyDeviceToHost, s), "score");
     check(cudaStreamSynchronize(s), "refine4");

@@ -78,7 +78,7 @@ __device__ bool may_contain(const DomainView& d, double row, double col, double 
 }
 
 // ------------------------------------------------------- FP32 pair arithmetic
-struct F2 {
+struct __align__(8) F2 {  // stored as one 8-byte word
   float hi, lo;
 };
 __device__ __forceinline__ F2 f2(float x) { return F2{x, 0.f}; }
@@ -1108,10 +1108,49 @@ __global__ void dedup_kernel(DedupArgs a) {
 // pair additions a lane instead of 95, and the warps' partials are added by
 // one warp per value instead of one warp for all.  (Pair addition is
 // commutative to the bit, and adding a zero pair changes nothing.)
+// The threads may be spread over the C blocks of a cluster (the warps of
+// block r follow those of block r - 1): a warp writes its partials into
+// every block's shared memory, so each block has the totals and goes on by
+// itself, and one cluster barrier separates the passes (two buffers: a block
+// may be one pass ahead of a reader).
 template <int K> struct BlockTotals {
-  F2 part[K][16];  // by value and warp
+  F2 part[2][K][16];  // by value and warp
   F2 total[K];
 };
+
+template <int C> __device__ __forceinline__ int team_rank() {
+  if (C == 1) return 0;
+  uint32_t r;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return int(r);
+}
+// This thread's number among the C blocks' threads, and their count.
+template <int C> __device__ __forceinline__ int team_thread() { return team_rank<C>() * int(blockDim.x) + int(threadIdx.x); }
+template <int C> __device__ __forceinline__ int team_size() { return C * int(blockDim.x); }
+template <int C> __device__ __forceinline__ void team_sync() {
+  if (C == 1) {
+    __syncthreads();
+    return;
+  }
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Stores a pair at the same place of every block's shared memory.
+template <int C> __device__ __forceinline__ void team_store(F2* p, F2 v) {
+  static_assert(alignof(F2) == 8, "one vector store per pair");
+  if (C == 1) {
+    *p = v;
+    return;
+  }
+  const uint32_t at = uint32_t(__cvta_generic_to_shared(p));
+#pragma unroll
+  for (int r = 0; r < C; ++r)
+    asm volatile(
+        "{\n .reg .b32 a;\n mapa.shared::cluster.u32 a, %0, %1;\n st.shared::cluster.v2.f32 [a], {%2, %3};\n}\n" ::"r"(
+            at),
+        "r"(r), "f"(v.hi), "f"(v.lo)
+        : "memory");
+}
 
 template <int N> struct LaneFold {
   // x: N values of which this lane's subset holds `count`; halves them
@@ -1139,20 +1178,23 @@ template <> struct LaneFold<1> {
   }
 };
 
-template <int K> __device__ __forceinline__ void block_total(const float (&v)[K], BlockTotals<K>& s) {
+template <int C = 1, int K>
+__device__ __forceinline__ void block_total(const float (&v)[K], BlockTotals<K>& s, int buffer = 0) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   F2 x[K];
 #pragma unroll
   for (int k = 0; k < K; ++k) x[k] = f2(v[k]);
   int index = 0, count = K;
   const F2 mine = LaneFold<K>::run(x, 16, index, count);
-  if (count > 0) s.part[index][warp] = mine;
-  __syncthreads();
-  for (int k = warp; k < K; k += nw) {
-    F2 y = lane < nw ? s.part[k][lane] : F2{0.f, 0.f};
-    for (int o = nw >> 1; o > 0; o >>= 1)
+  if (count > 0) team_store<C>(&s.part[buffer][index][team_rank<C>() * nw + warp], mine);
+  team_sync<C>();
+  const int parts = C * nw, per = 32 / parts, sub = lane % parts;  // partials per value, values per warp
+  for (int k0 = warp * per; k0 < K; k0 += nw * per) {
+    const int k = k0 + lane / parts;
+    F2 y = k < K ? s.part[buffer][k][sub] : F2{0.f, 0.f};
+    for (int o = parts >> 1; o > 0; o >>= 1)
       y = f2_add(y, F2{__shfl_down_sync(0xffffffffu, y.hi, o), __shfl_down_sync(0xffffffffu, y.lo, o)});
-    if (lane == 0) s.total[k] = y;
+    if (sub == 0 && k < K) s.total[k] = y;
   }
   __syncthreads();
 }
@@ -1278,14 +1320,14 @@ __device__ __forceinline__ float pair_score(F2 sum, F2 sq, F2 dot, int n, int ab
 // sum w q.  Six samples per step, all loads issued before the arithmetic
 // (four 0.164 and 0.336 ms at 2048^2 and over a full circle, six 0.162 and
 // 0.324, eight with fewer blocks 0.163 and 0.367); each thread still adds its
-// samples in order s, s + blockDim.x, ...
+// samples in order first, first + stride, ...
 constexpr int kScoreUnroll = 6;
-template <int Bits>
+constexpr int kTeamUnroll = 8;  // passes of a cluster: more registers per thread
+template <int Bits, int Unroll>
 __device__ __forceinline__ void inside_sums(const ImageView& img, const OriginalView& orig, const LocalPose& L,
-                                            float offset, float (&acc)[4]) {
-  constexpr int U = kScoreUnroll;
-  const int stride = blockDim.x;
-  for (int s0 = threadIdx.x; s0 < orig.n; s0 += U * stride) {
+                                            float offset, int first, int stride, float (&acc)[4]) {
+  constexpr int U = Unroll;
+  for (int s0 = first; s0 < orig.n; s0 += U * stride) {
     float4 p[U];
     float fy[U], fx[U];
     RawCell<Bits> raw[U];
@@ -1315,9 +1357,9 @@ __device__ __forceinline__ void inside_sums(const ImageView& img, const Original
 
 // continuous() of src/ncc_matching/matcher.cpp:144-156 at a level-local pose;
 // every thread of the block calls it and gets the score.
-template <int Bits>
+template <int Bits, int C = 1>
 __device__ __forceinline__ double continuous_pass(const ImageView& img, const OriginalView& orig, const LocalPose& lp,
-                                                  int absolute, BlockTotals<4>& tot) {
+                                                  int absolute, BlockTotals<4>& tot, int buffer = 0) {
   const LocalPose L = lp;
   const float hmax = float(img.h - 1 - L.R0), wmax = float(img.w - 1 - L.C0);
   const float hmin = float(-L.R0), wmin = float(-L.C0);
@@ -1333,9 +1375,9 @@ __device__ __forceinline__ double continuous_pass(const ImageView& img, const Or
   }
   float acc[4] = {0.f, 0.f, 0.f, 0.f};  // sum q, sum q^2, sum w q, out-of-image flag
   if (samples_inside(L, orig, hmin, hmax, wmin, wmax)) {
-    inside_sums<Bits>(img, orig, L, offset, acc);
+    inside_sums<Bits, C == 1 ? kScoreUnroll : kTeamUnroll>(img, orig, L, offset, team_thread<C>(), team_size<C>(), acc);
   } else
-  for (int s = threadIdx.x; s < orig.n; s += blockDim.x) {
+  for (int s = team_thread<C>(); s < orig.n; s += team_size<C>()) {
     const float dr = __ldg(orig.dr + s), dc = __ldg(orig.dc + s), w = __ldg(orig.w + s);
     const float y = L.fr + (L.ca * dr - L.sa * dc), x = L.fc + (L.sa * dr + L.ca * dc);
     if (!(y >= hmin && x >= wmin && y <= hmax && x <= wmax)) {
@@ -1349,7 +1391,7 @@ __device__ __forceinline__ double continuous_pass(const ImageView& img, const Or
     acc[1] = fmaf(q, q, acc[1]);
     acc[2] = fmaf(w, q, acc[2]);
   }
-  block_total<4>(acc, tot);
+  block_total<C>(acc, tot, buffer);
   bool ok = false;
   const float sc = tot.total[3].hi > 0 ? -INFINITY
                                        : pair_score(tot.total[0], tot.total[1], tot.total[2], orig.n, absolute, &ok);
@@ -1451,13 +1493,13 @@ struct SimSample {
 
 // Calls use(weight, inside, sample) for this thread's samples in order; four
 // samples' loads are issued before their arithmetic.
-template <class T, class Use>
+template <class T, int C = 1, class Use>
 __device__ __forceinline__ void sim_samples(const PixelView& img, const OriginalView& orig, const SimLocal& l, Use use) {
-  constexpr int U = 4;
+  constexpr int U = C == 1 ? 4 : kTeamUnroll;
   const T* __restrict__ v = static_cast<const T*>(img.v);
   const float hmin = float(-l.R0), wmin = float(-l.C0), hmax = float(img.h - 1 - l.R0), wmax = float(img.w - 1 - l.C0);
-  const int stride = blockDim.x;
-  for (int s0 = threadIdx.x; s0 < orig.n; s0 += U * stride) {
+  const int stride = team_size<C>();
+  for (int s0 = team_thread<C>(); s0 < orig.n; s0 += U * stride) {
     float4 p[U];
     float fy[U], fx[U], uu[U], vv[U];
     uint32_t raw[U][4];
@@ -1538,7 +1580,7 @@ template <class T> __global__ void __launch_bounds__(kAdjointThreads) adjoint_ke
       acc[11 + j] = fmaf(w, s.g[j], acc[11 + j]);
     }
   });
-  block_total<17>(acc, tot);
+  block_total(acc, tot);
   if (threadIdx.x < 4) {
     const F2* t = tot.total;
     const int j = threadIdx.x;
@@ -1565,16 +1607,16 @@ template <class T> __global__ void __launch_bounds__(kAdjointThreads) adjoint_ke
 // 25 w, 26 outside, with g = dq / d(row, col, angle, scale).
 constexpr int kSimSums = 27;
 
-template <class T>
+template <class T, int C>
 __device__ __noinline__ void sim_pass(const Refine4Args& a, SimLocal& loc, const double* pose,
-                                      BlockTotals<kSimSums>& tot) {
+                                      BlockTotals<kSimSums>& tot, int buffer) {
   if (threadIdx.x < 32) set_sim<T>(loc, a.img, a.orig, pose);
   __syncthreads();
   const SimLocal l = loc;
   float acc[kSimSums];
 #pragma unroll
   for (int j = 0; j < kSimSums; ++j) acc[j] = 0.f;
-  sim_samples<T>(a.img, a.orig, l, [&](float w, bool in, const SimSample& s) {
+  sim_samples<T, C>(a.img, a.orig, l, [&](float w, bool in, const SimSample& s) {
     acc[25] += w;
     if (!in) {
       acc[26] = 1.f;
@@ -1593,17 +1635,18 @@ __device__ __noinline__ void sim_pass(const Refine4Args& a, SimLocal& loc, const
       for (int j = i; j < 4; ++j, ++at) acc[at] = fmaf(s.g[i], s.g[j], acc[at]);
     }
   });
-  block_total<kSimSums>(acc, tot);
+  block_total<C>(acc, tot, buffer);
 }
 
 // The score alone: totals of 0 q, 1 q^2, 2 w q, 3 w, 4 outside.
-template <class T>
-__device__ __noinline__ double sim_score(const Refine4Args& a, SimLocal& loc, const double* pose, BlockTotals<5>& tot) {
+template <class T, int C>
+__device__ __noinline__ double sim_score(const Refine4Args& a, SimLocal& loc, const double* pose, BlockTotals<5>& tot,
+                                         int buffer) {
   if (threadIdx.x < 32) set_sim<T>(loc, a.img, a.orig, pose);
   __syncthreads();
   const SimLocal l = loc;
   float acc[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-  sim_samples<T>(a.img, a.orig, l, [&](float w, bool in, const SimSample& s) {
+  sim_samples<T, C>(a.img, a.orig, l, [&](float w, bool in, const SimSample& s) {
     acc[3] += w;
     if (!in) {
       acc[4] = 1.f;
@@ -1613,7 +1656,7 @@ __device__ __noinline__ double sim_score(const Refine4Args& a, SimLocal& loc, co
     acc[1] = fmaf(s.q, s.q, acc[1]);
     acc[2] = fmaf(w, s.q, acc[2]);
   });
-  block_total<5>(acc, tot);
+  block_total<C>(acc, tot, buffer);
   const F2* t = tot.total;
   const double n = double(a.orig.n);
   const double sq = pair_double(t[0]), sqq = pair_double(t[1]), swq = pair_double(t[2]), sw = pair_double(t[3]);
@@ -1628,24 +1671,27 @@ __device__ __noinline__ double sim_score(const Refine4Args& a, SimLocal& loc, co
 // the reference's refinement_step), an FP64 Gauss-Jordan solve with partial
 // pivoting (a matrix entry per lane of warp 0), the step clipped to the
 // limits, and up to four halvings; a step is taken only when the score
-// strictly increases.  64 poses of a 161^2 template: 2.29 -> 1.80 ms
-// (3000x4096 image).
-constexpr int kRefine4Threads = 256;
+// strictly increases.  64 poses of a 161^2 template: 2.29 -> 1.52 ms
+// (3000x4096 image; 1.80 with one block per pose).
+constexpr int kRefine4Threads = 256;  // of a team of C blocks
 
-template <class T>
-__global__ void __launch_bounds__(kRefine4Threads) refine4_kernel(const __grid_constant__ Refine4Args a) {
+template <class T, int C>
+__global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kRefine4Threads / C)
+    refine4_kernel(const __grid_constant__ Refine4Args a) {
   __shared__ BlockTotals<kSimSums> tot;
   __shared__ BlockTotals<5> tot5;
   __shared__ SimLocal loc;
   __shared__ double s_pose[4], s_try[4], s_delta[4], s_score, s_factor;
   __shared__ int s_go;
-  const int k = blockIdx.x, tid = threadIdx.x;
+  const int k = blockIdx.x / C, tid = threadIdx.x;
+  int pass = 0;
   if (tid < 4) s_pose[tid] = a.poses[4 * k + tid];
+  team_sync<C>();  // every block of the cluster runs and has read the pose
   double score = -INFINITY;
   const double n = double(a.orig.n);
   for (int it = 0; it <= a.iterations; ++it) {
     __syncthreads();
-    sim_pass<T>(a, loc, s_pose, tot);
+    sim_pass<T, C>(a, loc, s_pose, tot, pass++ & 1);
     if (tid < 32) {
       const F2* t = tot.total;
       const double sq = pair_double(t[0]), sqq = pair_double(t[1]), swq = pair_double(t[2]), sw = pair_double(t[25]);
@@ -1718,7 +1764,7 @@ __global__ void __launch_bounds__(kRefine4Threads) refine4_kernel(const __grid_c
     for (int bt = 0; bt < 4 && !accepted; ++bt) {
       if (tid < 4) s_try[tid] = s_pose[tid] + ldexp(s_factor, -bt) * s_delta[tid];
       __syncthreads();
-      const double got = sim_score<T>(a, loc, s_try, tot5);
+      const double got = sim_score<T, C>(a, loc, s_try, tot5, pass++ & 1);
       if (got > score) {
         accepted = true;
         if (tid < 4) s_pose[tid] = s_try[tid];
@@ -1734,11 +1780,12 @@ __global__ void __launch_bounds__(kRefine4Threads) refine4_kernel(const __grid_c
     __syncthreads();
     if (!s_go) {
       // converged: the score at the final pose
-      score = sim_score<T>(a, loc, s_pose, tot5);
+      score = sim_score<T, C>(a, loc, s_pose, tot5, pass++ & 1);
       break;
     }
   }
   __syncthreads();
+  if (team_rank<C>() != 0) return;
   if (tid < 4) a.poses[4 * k + tid] = s_pose[tid];
   if (tid == 0) a.score[k] = score;
 }
@@ -2133,6 +2180,10 @@ __global__ void __launch_bounds__(kSelectThreads) select_kernel(SelectArgs a) {
 }
 
 // --------------------------------------------------------------- refinement
+// A candidate is refined by 512 threads: one block, or a cluster of four
+// blocks whose SMs share the samples and which each follow the fit.
+constexpr int kRefineThreads = 512;
+
 // State of a block's fit.  Poses are {row, column, angle}; scalar FP64 work
 // is done by warp 0, a pose component per lane, and read by all threads
 // after a barrier.
@@ -2143,9 +2194,9 @@ struct FitShared {
   double pose[3], trial[3], seed[3], best[3];
   double delta[3], gn_delta[3], next_delta[3];
   double gscore, factor;  // score seen by the last Gauss-Newton pass (-inf if none); step factor
+  int buffer;             // of the next block total
   int ok, flag;           // result of the last Gauss-Newton pass; a decision of warp 0
-  float wbest[32];
-  int word[32];
+  F2 wbest[16];           // recovery search: {score, order} by warp
   double best_score;
 };
 
@@ -2156,7 +2207,7 @@ struct FitShared {
 // f.gn_delta hold the result, for every thread.  Kept out of line: its code
 // runs once per pass and is called from several places, and copies of it
 // would miss the instruction cache.
-template <int Bits>
+template <int Bits, int C>
 __device__ __noinline__ void gn_pass(const RefineArgs& a, FitShared& f, bool use_minimum, double minimum) {
   const ImageView& img = a.img;
   const OriginalView& orig = a.orig;
@@ -2178,11 +2229,11 @@ __device__ __noinline__ void gn_pass(const RefineArgs& a, FitShared& f, bool use
 #pragma unroll
   for (int k = 0; k < 19; ++k) acc[k] = 0.f;
   const bool inside = samples_inside(L, orig, hmin, hmax, wmin, wmax);
-  const int stride = blockDim.x;
-  // four samples per step, all loads issued before the arithmetic; each
-  // thread still adds its samples in order s, s + blockDim.x, ...
-  constexpr int U = 4;
-  for (int s0 = threadIdx.x; s0 < orig.n; s0 += U * stride) {
+  const int stride = team_size<C>();
+  // U samples per step, all loads issued before the arithmetic; each
+  // thread still adds its samples in order s, s + stride, ...
+  constexpr int U = C == 1 ? 4 : kTeamUnroll;
+  for (int s0 = team_thread<C>(); s0 < orig.n; s0 += U * stride) {
     float4 p[U];
     float fy[U], fx[U];
     RawCell<Bits> raw[U];
@@ -2233,8 +2284,9 @@ __device__ __noinline__ void gn_pass(const RefineArgs& a, FitShared& f, bool use
       acc[17] = fmaf(g2, g2, acc[17]);
     }
   }
-  block_total<19>(acc, f.tot19);
+  block_total<C>(acc, f.tot19, f.buffer);
   if (threadIdx.x < 32) {
+    if (threadIdx.x == 0) f.buffer ^= 1;
     // every lane evaluates the scalar terms, lane l < axes (axes + 1) one
     // matrix or right-hand-side entry (row l / (axes + 1)), which it carries
     // through the elimination
@@ -2311,8 +2363,11 @@ __device__ __forceinline__ void local_pose(const RefineArgs& a, FitShared& f, co
 }
 
 // Score at the pose in f.lp, for every thread.
-template <int Bits> __device__ __noinline__ double score_pass(const RefineArgs& a, FitShared& f) {
-  return continuous_pass<Bits>(a.img, a.orig, f.lp, a.absolute, f.tot4);
+template <int Bits, int C> __device__ __noinline__ double score_pass(const RefineArgs& a, FitShared& f) {
+  const double score = continuous_pass<Bits, C>(a.img, a.orig, f.lp, a.absolute, f.tot4, f.buffer);
+  if (threadIdx.x == 0) f.buffer ^= 1;
+  __syncthreads();
+  return score;
 }
 
 // The step's factor from f.delta (warp 0): at most .75 rows and columns and
@@ -2354,14 +2409,14 @@ __device__ __forceinline__ void trial_pose(const RefineArgs& a, FitShared& f, in
 // fit() of src/ncc_matching/matcher.cpp:903-982 for the pose in f.pose with
 // score `score` (single-model query: no memo, no background guard); returns
 // the fitted pose's score.
-template <int Bits> __device__ __noinline__ double fit_full(const RefineArgs& a, FitShared& f, double score) {
+template <int Bits, int C> __device__ __noinline__ double fit_full(const RefineArgs& a, FitShared& f, double score) {
   if (!a.subpixel) return score;
   bool cached = false;  // f.next_delta is the step at f.pose
   for (int it = 0; it < 6; ++it) {
     if (!cached) {
       if (threadIdx.x < 32) local_pose(a, f, f.pose);
       __syncthreads();
-      gn_pass<Bits>(a, f, false, 0.);
+      gn_pass<Bits, C>(a, f, false, 0.);
       if (!f.ok) break;
     }
     bool accepted = false, next_valid = false;
@@ -2380,14 +2435,14 @@ template <int Bits> __device__ __noinline__ double fit_full(const RefineArgs& a,
       if (!f.flag) continue;
       double got;
       if (bt == 0 && it + 1 < 6) {
-        gn_pass<Bits>(a, f, true, score);
+        gn_pass<Bits, C>(a, f, true, score);
         got = f.gscore;
         next_valid = f.ok;
         if (threadIdx.x < 3) f.next_delta[threadIdx.x] = f.gn_delta[threadIdx.x];
-        if (!isfinite(got)) got = score_pass<Bits>(a, f);
+        if (!isfinite(got)) got = score_pass<Bits, C>(a, f);
       } else {
         next_valid = false;
-        got = score_pass<Bits>(a, f);
+        got = score_pass<Bits, C>(a, f);
       }
       if (got > score) {
         score = got;
@@ -2406,12 +2461,12 @@ template <int Bits> __device__ __noinline__ double fit_full(const RefineArgs& a,
 }
 
 // refine_coarse_candidate of src/ncc_matching/matcher.cpp:853-877
-template <int Bits> __device__ __noinline__ double fit_coarse(const RefineArgs& a, FitShared& f, double score) {
+template <int Bits, int C> __device__ __noinline__ double fit_coarse(const RefineArgs& a, FitShared& f, double score) {
   if (!a.subpixel) return score;
   for (int it = 0; it < 6; ++it) {
     if (threadIdx.x < 32) local_pose(a, f, f.pose);
     __syncthreads();
-    gn_pass<Bits>(a, f, false, 0.);
+    gn_pass<Bits, C>(a, f, false, 0.);
     if (!f.ok) break;
     bool accepted = false;
     for (int bt = 0; bt < 4 && !accepted; ++bt) {
@@ -2426,7 +2481,7 @@ template <int Bits> __device__ __noinline__ double fit_coarse(const RefineArgs& 
       }
       __syncthreads();
       if (!f.flag) continue;
-      const double got = score_pass<Bits>(a, f);
+      const double got = score_pass<Bits, C>(a, f);
       if (got > score) {
         score = got;
         accepted = true;
@@ -2443,8 +2498,8 @@ template <int Bits> __device__ __noinline__ double fit_coarse(const RefineArgs& 
 // Discrete level-0 search around the seed (matcher.cpp:986-1059): one warp per
 // (patch, position), exact integer moments in the loop.  Leaves the first
 // strict maximum over (patch order, dr, dc) in f.best and f.best_score (-inf if none).
-__device__ __noinline__ void recovery_search(const RefineArgs& a, FitShared& f) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+template <int C> __device__ __noinline__ void recovery_search(const RefineArgs& a, FitShared& f) {
+  const int lane = threadIdx.x & 31, warp = team_thread<C>() >> 5, nw = team_size<C>() >> 5;
   const double seed_row = f.seed[0], seed_col = f.seed[1], seed_angle = f.seed[2];
   float best = -INFINITY;
   int border = INT32_MAX;
@@ -2490,18 +2545,15 @@ __device__ __noinline__ void recovery_search(const RefineArgs& a, FitShared& f) 
     }
     ++k;
   }
-  if (lane == 0) {
-    f.wbest[warp] = best;
-    f.word[warp] = border;
-  }
-  __syncthreads();
+  if (lane == 0) team_store<C>(&f.wbest[warp], F2{best, __int_as_float(border)});
+  team_sync<C>();
   if (threadIdx.x == 0) {
     float bs = -INFINITY;
     int bo = INT32_MAX;
     for (int w = 0; w < nw; ++w)
-      if (better(f.wbest[w], f.word[w], bs, bo)) {
-        bs = f.wbest[w];
-        bo = f.word[w];
+      if (better(f.wbest[w].hi, __float_as_int(f.wbest[w].lo), bs, bo)) {
+        bs = f.wbest[w].hi;
+        bo = __float_as_int(f.wbest[w].lo);
       }
     f.best[0] = seed_row;
     f.best[1] = seed_col;
@@ -2527,31 +2579,31 @@ __device__ __noinline__ void recovery_search(const RefineArgs& a, FitShared& f) 
   __syncthreads();
 }
 
-constexpr int kRefineThreads = 512;
-
 // refine_candidate (src/ncc_matching/matcher.cpp:878-1061) for one queued
 // candidate per block.  Bound by the latency of a chain of passes: gathers,
 // two reductions and FP64 algebra each.  Five 128^2 candidates (six
-// Gauss-Newton passes and four scores each): 0.385 -> 0.177 ms (19 shuffle trees
+// Gauss-Newton passes and four scores each): 0.385 -> 0.164 ms (19 shuffle trees
 // per warp and once more on warp 0, FP64 steps on one thread, one sample at a
 // time before).
-template <int Bits>
-__global__ void __launch_bounds__(kRefineThreads) refine_kernel(const __grid_constant__ RefineArgs a) {
+template <int Bits, int C>
+__global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kRefineThreads / C)
+    refine_kernel(const __grid_constant__ RefineArgs a) {
   __shared__ FitShared f;
-  const int b = blockIdx.x;
+  const int b = blockIdx.x / C;
   // a queued round after the end of the selection has nothing to refine
   if (a.batch_count < 0 && a.state->done) return;
   if (b >= (a.batch_count >= 0 ? a.batch_count : a.state->batch_count)) return;
   const int i = a.batch[b], t = threadIdx.x;
   double score = a.sorted[i].score;
   if (t < 3) f.pose[t] = f.seed[t] = (&a.sorted[i].row)[t];
-  __syncthreads();
+  if (t == 0) f.buffer = 0;
+  team_sync<C>();  // every block of the cluster runs
   if (a.finest) {
-    score = fit_coarse<Bits>(a, f, score);
+    score = fit_coarse<Bits, C>(a, f, score);
   } else {
-    score = fit_full<Bits>(a, f, score);
+    score = fit_full<Bits, C>(a, f, score);
     if (a.subpixel && a.top > 0 && score < a.min_score) {
-      recovery_search(a, f);
+      recovery_search<C>(a, f);
       // the search starts from the fitted candidate: only a strictly higher
       // discrete score moves it
       const bool move = f.best_score > score && (f.best[0] != f.pose[0] || f.best[1] != f.pose[1] || f.best[2] != f.pose[2]);
@@ -2564,8 +2616,8 @@ __global__ void __launch_bounds__(kRefineThreads) refine_kernel(const __grid_con
         }
         if (t < 32) local_pose(a, f, f.pose);
         __syncthreads();
-        score = score_pass<Bits>(a, f);
-        score = fit_full<Bits>(a, f, score);
+        score = score_pass<Bits, C>(a, f);
+        score = fit_full<Bits, C>(a, f, score);
         if (!(score > fitted)) {
           score = fitted;
           if (t < 3) f.pose[t] = f.seed[t];
@@ -2574,7 +2626,7 @@ __global__ void __launch_bounds__(kRefineThreads) refine_kernel(const __grid_con
       }
     }
   }
-  if (t == 0) {
+  if (t == 0 && team_rank<C>() == 0) {
     Refined r;
     Cand c{};
     r.row = c.row = f.pose[0];
@@ -2728,12 +2780,16 @@ cudaError_t launch_adjoint(const AdjointArgs& a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_refine4(const Refine4Args& a, cudaStream_t s) {
+cudaError_t launch_refine4(const Refine4Args& a, cudaStream_t s, int sms) {
   if (a.n <= 0) return cudaSuccess;
+  // few poses: four SMs share the samples of one; from about a pose per SM on
+  // the GPU is full and the cluster barriers only cost
+  const bool team = a.n < sms;
+  const int grid = team ? 4 * a.n : a.n, threads = team ? kRefine4Threads / 4 : kRefine4Threads;
   if (a.img.type == 1)
-    refine4_kernel<uint16_t><<<a.n, kRefine4Threads, 0, s>>>(a);
+    team ? refine4_kernel<uint16_t, 4><<<grid, threads, 0, s>>>(a) : refine4_kernel<uint16_t, 1><<<grid, threads, 0, s>>>(a);
   else
-    refine4_kernel<uint8_t><<<a.n, kRefine4Threads, 0, s>>>(a);
+    team ? refine4_kernel<uint8_t, 4><<<grid, threads, 0, s>>>(a) : refine4_kernel<uint8_t, 1><<<grid, threads, 0, s>>>(a);
   return cudaGetLastError();
 }
 
@@ -2794,12 +2850,25 @@ cudaError_t launch_select(const SelectArgs& a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_refine(const RefineArgs& a, int batch_limit, cudaStream_t s) {
+namespace {
+template <int C> void refine_launch(const RefineArgs& a, int batch_limit, cudaStream_t s) {
+  const int grid = C * batch_limit, threads = kRefineThreads / C;
   switch (a.img.bits) {
-    case 8: refine_kernel<8><<<batch_limit, kRefineThreads, 0, s>>>(a); break;
-    case 16: refine_kernel<16><<<batch_limit, kRefineThreads, 0, s>>>(a); break;
-    default: refine_kernel<0><<<batch_limit, kRefineThreads, 0, s>>>(a); break;
+    case 8: refine_kernel<8, C><<<grid, threads, 0, s>>>(a); break;
+    case 16: refine_kernel<16, C><<<grid, threads, 0, s>>>(a); break;
+    default: refine_kernel<0, C><<<grid, threads, 0, s>>>(a); break;
   }
+}
+}  // namespace
+
+cudaError_t launch_refine(const RefineArgs& a, int batch_limit, cudaStream_t s) {
+  // a large template's samples pay for the cluster's barriers: 128^2 0.182
+  // (one block) and 0.164 ms (cluster), 256^2 0.49 and 0.40, but 64^2 0.086
+  // and 0.097, 48^2 over a full circle 0.106 and 0.122
+  if (a.orig.n >= 12288)
+    refine_launch<4>(a, batch_limit, s);
+  else
+    refine_launch<1>(a, batch_limit, s);
   return cudaGetLastError();
 }
 

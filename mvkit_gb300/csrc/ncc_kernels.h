@@ -402,7 +402,7 @@ cudaError_t launch_track(const TrackArgs& a, int max_candidates, cudaStream_t s,
 cudaError_t launch_dedup(const DedupArgs& a, int max_candidates, cudaStream_t s);
 cudaError_t launch_score(const ScoreArgs& a, int max_candidates, cudaStream_t s, int sms);
 cudaError_t launch_adjoint(const AdjointArgs& a, cudaStream_t s);
-cudaError_t launch_refine4(const Refine4Args& a, cudaStream_t s);
+cudaError_t launch_refine4(const Refine4Args& a, cudaStream_t s, int sms);
 cudaError_t launch_sort(const SortArgs& a, int max_candidates, cudaStream_t s);
 int sort_launches(int max_candidates);  // kernels launch_sort queues
 cudaError_t launch_select(const SelectArgs& a, cudaStream_t s);
