@@ -76,7 +76,7 @@ struct TcPlan {
   size_t smem = 0;        // dynamic shared memory of the launch
   std::vector<TcGroup> groups;
   std::vector<int32_t> group_of_src;
-  std::vector<std::unique_ptr<DevBuf<uint8_t>>> weights;
+  DevBuf<uint8_t> weights;  // every group's chunks
 };
 
 struct DevLevel {
@@ -130,6 +130,29 @@ struct DevLevel {
     }
     desc.push_back(d);
     angles.push_back(r.angle);
+  }
+  // per patch: largest |weight|, and largest sum of |weight| over a row (filled on demand)
+  std::vector<std::pair<double, double>> weight_range;
+  std::pair<double, double> patch_weight_range(size_t i) {
+    for (size_t p = weight_range.size(); p <= i; ++p) weight_range.emplace_back(-1, -1);
+    if (weight_range[i].first < 0) {
+      const PatchDesc& d = desc[i];
+      double most = 0, row_most = 0, row = 0;
+      int at = INT32_MIN;
+      for (int32_t k = d.sample_off; k < d.sample_off + d.n; ++k) {
+        // samples are in row-major order
+        if ((offs[size_t(k)] >> 16) != at) {
+          at = offs[size_t(k)] >> 16;
+          row = 0;
+        }
+        const double x = std::abs(double(w[size_t(k)]));
+        most = std::max(most, x);
+        row += x;
+        row_most = std::max(row_most, row);
+      }
+      weight_range[i] = {most, row_most};
+    }
+    return weight_range[i];
   }
   // tensor-core plans of tracking steps into this level, by query plan
   std::map<std::vector<int32_t>, std::shared_ptr<const TcPlan>> tc_plans;
@@ -348,18 +371,6 @@ thread_local int t_tc_lookahead = 8;
 // launches are merged (0, default: every find launches its own).
 thread_local int t_merge_tc = 0;
 
-uint16_t half_bits(double x) {
-  const _Float16 h = static_cast<_Float16>(x);
-  uint16_t b;
-  std::memcpy(&b, &h, sizeof(b));
-  return b;
-}
-double half_value(uint16_t b) {
-  _Float16 h;
-  std::memcpy(&h, &b, sizeof(b));
-  return double(h);
-}
-
 // fp16 planes of level t: the level minus `offset` as base-64 digits, each
 // an exact fp16 integer: the first signed (|d| <= 2048), the others in
 // [0, 64) (parts 1: the value itself; 2: 64 h + l; up to 4 for uint16
@@ -442,17 +453,10 @@ bool lattice_exact32(double v) {
 // Builds the tensor-core groups of the tracking step into level T (query
 // plan `lp`, `nsrc` patches on the source level).  A group is the rotated
 // patches (origin on the lattice) of one source patch's selected list; the
-// sources with identical lists share it.  Weights: per chunk of rg grid
-// rows, an N x K fp16 matrix in the canonical K-major no-swizzle layout
-// (8 x 8 core matrices of 128 bytes, K-adjacent cores 128 bytes apart,
-// N-adjacent cores K/8 x 128 bytes apart); column (((p 5 + dc) rg + y mod
-// rg) 2 + half) holds the high or low fp16 half of sigma w_p(y, x - dc), row
-// x + part kw the same for each plane part (x 64 per digit above the last).
-// The slots of one output sit side by side, so 32 accumulator columns hold
-// 16 / rg whole outputs (rg is 1, 2 or 4).  The last 16 rows hold the
-// column's row sum for grid row y as two fp16 terms (x 64 likewise), which
-// the centring columns of the window multiply.
-std::shared_ptr<const TcPlan> build_tc_plan(const DevLevel& T, size_t nsrc, const LevelPlan& lp, int parts,
+// sources with identical lists share it.  The slots of one output sit side by
+// side in a chunk's columns, so 32 accumulator columns hold 16 / rg whole
+// outputs (rg is 1, 2 or 4).
+std::shared_ptr<const TcPlan> build_tc_plan(DevLevel& T, size_t nsrc, const LevelPlan& lp, int parts,
                                             float offset, size_t budget, int lookahead) {
   auto plan = std::make_shared<TcPlan>();
   plan->parts = parts;
@@ -569,105 +573,86 @@ std::shared_ptr<const TcPlan> build_tc_plan(const DevLevel& T, size_t nsrc, cons
   plan->stage_bytes = int(max_chunk);
   plan->abuf_bytes = int(per_row * size_t(rows));
   plan->smem = ring + 2 * per_row * size_t(rows);
+  // the weight chunks are filled on the device (tc_weights_kernel)
+  std::vector<TcWeightJob> jobs;
+  size_t bytes = 0, scratch_rows = 0;
+  auto chunk_elems = [&](const Proto& pr) { return size_t(pr.n) * size_t(parts * pr.kw + 16); };
+  for (const Proto& pr : protos) bytes += size_t((pr.kr + pr.rg - 1) / pr.rg) * chunk_elems(pr) * 2;
+  plan->weights.reserve(bytes);
+  check(cudaMemsetAsync(plan->weights.p, 0, bytes, nullptr), "tc weights");
+  size_t at = 0;
   for (const Proto& pr : protos) {
-    const int P = int(pr.descs.size()), K = parts * pr.kw + 16, N = pr.n;
-    const size_t chunk_elems = size_t(N) * size_t(K);
+    const int P = int(pr.descs.size());
     double maxw = 0, maxrow = 0;
     for (int32_t di : pr.descs) {
-      const PatchDesc& d = T.desc[size_t(di)];
-      std::vector<double> row(size_t(pr.kr), 0.0);
-      for (int i = 0; i < d.n; ++i) {
-        const double w = double(T.w[size_t(d.sample_off + i)]);
-        maxw = std::max(maxw, std::abs(w));
-        row[size_t((T.offs[size_t(d.sample_off + i)] >> 16) - pr.rmin)] += std::abs(w);
-      }
-      for (double r : row) maxrow = std::max(maxrow, r);
+      const auto range = T.patch_weight_range(size_t(di));
+      maxw = std::max(maxw, range.first);
+      maxrow = std::max(maxrow, range.second);
     }
     // weight scale: a power of two keeping the weights (x 64 for a split
     // level) and the centring row sums (x 64 likewise) within fp16 range
     const double m64 = std::ldexp(1.0, 6 * (parts - 1));  // multiplier of the first part
     const double limit = std::min(maxw > 0 ? 16384.0 / (maxw * m64) : 1e30, maxrow > 0 ? 16384.0 / (maxrow * m64) : 1e30);
     const double sigma = limit < 1e30 ? std::ldexp(1., int(std::floor(std::log2(limit)))) : 1.0;
-    const int rg = pr.rg, chunks = (pr.kr + rg - 1) / rg;
-    std::vector<uint16_t> host(size_t(chunks) * chunk_elems, 0);
     TcGroup g{};
+    g.b = plan->weights.p + at;
     g.kr = pr.kr;
     g.kw = pr.kw;
     g.parts = parts;
     g.rmin = pr.rmin;
     g.cmin = pr.cmin;
     g.p = P;
-    g.rg = rg;
-    g.n = N;
+    g.rg = pr.rg;
+    g.n = pr.n;
     g.rows_slab = rows;
     g.inv_scale = float(1.0 / sigma);
     g.macs = 0;
-    // element of grid row y, column (patch q, placement dc, half), K index k:
-    // chunk y / rg, N column ((q 5 + dc) rg + y mod rg) 2 + half
-    auto at = [&](size_t y, int q, int dc, int half, int k) {
-      const int n = ((q * 5 + dc) * rg + int(y % size_t(rg))) * 2 + half;
-      return (y / size_t(rg)) * chunk_elems + size_t(n / 8) * size_t(K / 8) * 64 + size_t(k / 8) * 64 +
-             size_t(n % 8) * 8 + size_t(k % 8);
-    };
     for (int q = 0; q < P; ++q) {
       const PatchDesc& d = T.desc[size_t(pr.descs[size_t(q)])];
-      double sum = 0;
-      std::vector<double> rs(size_t(pr.kr) * 2, 0.0);  // row sums of the two halves
-      for (int i = 0; i < d.n; ++i) {
-        const int32_t o = T.offs[size_t(d.sample_off + i)];
-        const int row = o >> 16, col = int(int16_t(o & 0xffff));
-        const double ws = double(T.w[size_t(d.sample_off + i)]) * sigma;
-        const uint16_t hi = half_bits(ws);
-        const double hv = half_value(hi);
-        const uint16_t lo = half_bits(ws - hv);
-        const double lv = half_value(lo);
-        sum += hv + lv;
-        const size_t y = size_t(row - pr.rmin);
-        rs[y * 2] += hv;
-        rs[y * 2 + 1] += lv;
-        for (int dc = 0; dc < 5; ++dc) {
-          const int x = col - pr.cmin + dc;
-          for (int part = 0; part < parts; ++part) {
-            const double mult = std::ldexp(1.0, 6 * (parts - 1 - part));
-            const int k = part * pr.kw + x;
-            for (int half = 0; half < 2; ++half)
-              host[at(y, q, dc, half, k)] = half_bits((half ? lv : hv) * mult);
-          }
-        }
-      }
-      // centring rows: the row sum of each column as two fp16 terms
-      double ecorr = 0;
-      const int kc0 = parts * pr.kw;
-      for (size_t y = 0; y < size_t(pr.kr); ++y)
-        for (int half = 0; half < 2; ++half) {
-          const double r = rs[y * 2 + size_t(half)];
-          const uint16_t f1 = half_bits(r);
-          const uint16_t f2 = half_bits(r - half_value(f1));
-          ecorr += half_value(f1) + half_value(f2);
-          // part q of the centre meets 64^(parts - 1 - q) x the row sum
-          for (int dc = 0; dc < 5; ++dc)
-            for (int part = 0; part < parts; ++part) {
-              const double mult = std::ldexp(1.0, 6 * (parts - 1 - part));
-              host[at(y, q, dc, half, kc0 + 2 * part)] = half_bits(mult * half_value(f1));
-              host[at(y, q, dc, half, kc0 + 2 * part + 1)] = half_bits(mult * half_value(f2));
-            }
-        }
-      g.ecorr[q] = float(ecorr / sigma);
+      TcWeightJob j{};
+      j.b = plan->weights.p + at;
+      j.chunk_elems = (long long)chunk_elems(pr);
+      j.sample_off = d.sample_off;
+      j.n = d.n;
+      j.rmin = pr.rmin;
+      j.cmin = pr.cmin;
+      j.kr = pr.kr;
+      j.kw = pr.kw;
+      j.parts = parts;
+      j.rg = pr.rg;
+      j.K = parts * pr.kw + 16;
+      j.q = q;
+      j.sigma = float(sigma);
+      j.rows_off = int(scratch_rows);
+      scratch_rows += 2 * size_t(pr.kr);
+      jobs.push_back(j);
       g.k_of[q] = pr.ks[size_t(q)];
       const int32_t o0 = T.offs[size_t(d.sample_off)];
       g.r0[q] = o0 >> 16;
       g.c0[q] = int(int16_t(o0 & 0xffff));
-      g.weff[q] = float(sum / sigma);
-      g.weff_k[pr.ks[size_t(q)]] = g.weff[q];
       g.macs += 25ll * d.n;
     }
-    auto buf = std::make_unique<DevBuf<uint8_t>>();
-    buf->reserve(host.size() * 2);
-    check(cudaMemcpy(buf->p, host.data(), host.size() * 2, cudaMemcpyHostToDevice), "tc weights");
-    g.b = buf->p;
-    plan->weights.push_back(std::move(buf));
+    at += size_t((pr.kr + pr.rg - 1) / pr.rg) * chunk_elems(pr) * 2;
     plan->groups.push_back(g);
   }
+  DevBuf<TcWeightJob> d_jobs;
+  DevBuf<TcWeightSums> d_sums;
+  DevBuf<unsigned long long> d_rows;
+  d_jobs.upload(jobs, nullptr);
+  d_sums.reserve(jobs.size());
+  d_rows.reserve(scratch_rows);
+  check(cudaMemsetAsync(d_rows.p, 0, scratch_rows * sizeof(unsigned long long), nullptr), "tc weights");
+  check(launch_tc_weights(d_jobs.p, int(jobs.size()), T.d_sw.p, d_rows.p, d_sums.p, nullptr), "tc weights");
+  std::vector<TcWeightSums> sums(jobs.size());
+  check(cudaMemcpy(sums.data(), d_sums.p, sums.size() * sizeof(TcWeightSums), cudaMemcpyDeviceToHost), "tc weights");
+  size_t job = 0;
+  for (TcGroup& g : plan->groups)
+    for (int q = 0; q < g.p; ++q, ++job) {
+      const double unit = std::ldexp(1., -24), sigma = double(jobs[job].sigma);
+      g.ecorr[q] = float(double(sums[job].ecorr) * unit / sigma);
+      g.weff[q] = float(double(sums[job].sum) * unit / sigma);
+      g.weff_k[g.k_of[q]] = g.weff[q];
+    }
   return plan;
 }
 

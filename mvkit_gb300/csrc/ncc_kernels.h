@@ -231,6 +231,24 @@ __device__ __forceinline__ float tc_plane_offset(float fixed, const QueryState* 
 }
 #endif
 size_t tc_kernel_static_smem();
+
+// Weight matrix part of one patch of a group (launch_tc_weights).
+struct TcWeightJob {
+  uint8_t* b;                            // the group's chunks
+  long long chunk_elems;                 // N x K
+  int sample_off, n;                     // the patch's samples
+  int rmin, cmin, kr, kw, parts, rg, K;  // the group's shape
+  int q;                                 // the patch's index in the group
+  float sigma;                           // weight scale (a power of two)
+  int rows_off;                          // first row of its 2 kr row sums in the scratch
+};
+struct TcWeightSums {
+  long long sum, ecorr;                  // of the fp16 weights and of the centring row sums, in units of 2^-24
+};
+// Fills the (zeroed) weight chunks of every job and its sums; `rows`: zeroed
+// scratch, 2 kr entries per job at rows_off.
+cudaError_t launch_tc_weights(const TcWeightJob* jobs, int njobs, const int2* sw, unsigned long long* rows,
+                              TcWeightSums* sums, cudaStream_t s);
 // Groups the step's candidates into tiles (counts, tile list, order).
 cudaError_t launch_tc_group(const TcArgs& a, int ngroups, int32_t* counts, int32_t* offsets, int32_t* cursor,
                             int max_candidates, cudaStream_t s);

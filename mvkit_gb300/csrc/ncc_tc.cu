@@ -745,6 +745,69 @@ __global__ void tc_planes_kernel(LevelImage lev, __half* planes, int pitch, floa
   }
 }
 
+// Weight chunks of a group, one block per (group, patch): a chunk of rg grid
+// rows is an N x K fp16 matrix in the canonical K-major no-swizzle layout
+// (8 x 8 core matrices of 128 bytes, K-adjacent cores 128 bytes apart,
+// N-adjacent cores K/8 x 128 bytes apart); column (((q 5 + dc) rg + y mod rg)
+// 2 + half) holds the high or low fp16 half of sigma w_q(y, x - dc), row
+// x + part kw the same for each plane part (x 64 per digit above the last).
+// The last 16 rows hold the column's row sum for grid row y as two fp16 terms
+// (x 64 likewise), which the centring columns of the window multiply.  The
+// halves are multiples of 2^-24, so the sums are added as integers: any order
+// gives the same.  A 128^2 template's three plans (270 patches of 90 groups
+// at the finest): 76 -> 1.5 ms with the host's work around it (on the host before).
+__global__ void __launch_bounds__(256) tc_weights_kernel(const TcWeightJob* jobs, const int2* __restrict__ sw,
+                                                         unsigned long long* rows, TcWeightSums* sums) {
+  const TcWeightJob J = jobs[blockIdx.x];
+  __shared__ unsigned long long s_sum, s_ecorr;
+  if (threadIdx.x == 0) s_sum = s_ecorr = 0;
+  __half* out = reinterpret_cast<__half*>(J.b);
+  unsigned long long* rs = rows + J.rows_off;
+  auto at = [&](int y, int dc, int half, int k) {
+    const int n = ((J.q * 5 + dc) * J.rg + y % J.rg) * 2 + half;
+    return size_t(y / J.rg) * size_t(J.chunk_elems) + size_t(n / 8) * size_t(J.K / 8) * 64 + size_t(k / 8) * 64 +
+           size_t((n % 8) * 8 + k % 8);
+  };
+  for (int i = threadIdx.x; i < J.n; i += blockDim.x) {
+    const int2 o = __ldg(sw + J.sample_off + i);
+    const int y = (o.x >> 16) - J.rmin, x = int(int16_t(o.x & 0xffff)) - J.cmin;
+    const float ws = __fmul_rn(__int_as_float(o.y), J.sigma);  // exact
+    const float hv = __half2float(__float2half_rn(ws));
+    const float lv = __half2float(__float2half_rn(__fsub_rn(ws, hv)));  // the difference is exact
+    atomicAdd(rs + 2 * y, (unsigned long long)__float2ll_rn(hv * 16777216.f));
+    atomicAdd(rs + 2 * y + 1, (unsigned long long)__float2ll_rn(lv * 16777216.f));
+    for (int part = 0; part < J.parts; ++part) {
+      const float mult = float(1 << (6 * (J.parts - 1 - part)));
+      const __half h = __float2half_rn(hv * mult), l = __float2half_rn(lv * mult);
+      for (int dc = 0; dc < 5; ++dc) {
+        out[at(y, dc, 0, part * J.kw + x + dc)] = h;
+        out[at(y, dc, 1, part * J.kw + x + dc)] = l;
+      }
+    }
+  }
+  __threadfence();
+  __syncthreads();
+  const int kc0 = J.parts * J.kw;
+  for (int i = threadIdx.x; i < 2 * J.kr; i += blockDim.x) {
+    const long long units = (long long)__ldcg(rs + i);
+    const double r = double(units) * 5.9604644775390625e-8;  // 2^-24
+    const double f1 = double(__half2float(__double2half(r)));
+    const double f2 = double(__half2float(__double2half(r - f1)));
+    atomicAdd(&s_sum, (unsigned long long)units);
+    atomicAdd(&s_ecorr, (unsigned long long)__double2ll_rn((f1 + f2) * 16777216.));
+    for (int part = 0; part < J.parts; ++part) {
+      const double mult = double(1 << (6 * (J.parts - 1 - part)));
+      const __half h1 = __double2half(mult * f1), h2 = __double2half(mult * f2);
+      for (int dc = 0; dc < 5; ++dc) {
+        out[at(i / 2, dc, i & 1, kc0 + 2 * part)] = h1;
+        out[at(i / 2, dc, i & 1, kc0 + 2 * part + 1)] = h2;
+      }
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) sums[blockIdx.x] = TcWeightSums{(long long)s_sum, (long long)s_ecorr};
+}
+
 // Grouping of the step's candidates: counts per group, tile list, order.
 __global__ void tc_count_kernel(const Cand* in, const QueryState* state, int slot, const int32_t* group_of_src,
                                 int32_t* counts) {
@@ -858,6 +921,12 @@ cudaError_t launch_tc_group(const TcArgs& a, int ngroups, int32_t* counts, int32
   tc_count_kernel<<<blocks, 256, 0, s>>>(a.in, a.state, a.in_slot, a.group_of_src, counts);
   tc_plan_kernel<<<1, 1024, 0, s>>>(counts, ngroups, offsets, cursor, a.tiles, kTcMaxTiles);
   tc_scatter_kernel<<<blocks, 256, 0, s>>>(a.in, a.state, a.in_slot, a.group_of_src, offsets, cursor, a.order);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_tc_weights(const TcWeightJob* jobs, int njobs, const int2* sw, unsigned long long* rows,
+                              TcWeightSums* sums, cudaStream_t s) {
+  if (njobs > 0) tc_weights_kernel<<<njobs, 256, 0, s>>>(jobs, sw, rows, sums);
   return cudaGetLastError();
 }
 
