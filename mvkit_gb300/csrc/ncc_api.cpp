@@ -80,24 +80,21 @@ struct TcPlan {
 };
 
 struct DevLevel {
-  int32_t lin_pitch = 0, lin_rows = 0;  // staged tracking window geometry
+  int32_t lin_rows = 0;             // rows and columns of a tracking window that holds any 5x5 placement set
   std::vector<PatchDesc> desc;      // host copy (model patches + query endpoints)
   std::vector<double> angles;
   size_t model_patches = 0;         // trained patches; endpoints follow
   std::vector<int32_t> offs, runs, runs_end;
   std::vector<float> w;
-  std::vector<int2> sw, lw;
   DevBuf<PatchDesc> d_desc;
-  DevBuf<int32_t> d_offs, d_runs, d_runs_end;
   DevBuf<float> d_w;
-  DevBuf<int2> d_sw, d_lw;
+  DevBuf<int2> d_sw;
   DevBuf<int4> d_run4;
   // Window geometry for a level of width x height: any rotation's raster
   // fits the diagonal; 5x5 placements and centre rounding add 8 cells.
   void set_geometry(size_t width, size_t height) {
     const int diag = int(std::ceil(std::hypot(double(width), double(height)))) + 1;
     lin_rows = diag + 8;
-    lin_pitch = lin_rows + ((5 - lin_rows) % 32 + 32) % 32;
   }
   void append(const Raster& r) {
     PatchDesc d{};
@@ -115,12 +112,8 @@ struct DevLevel {
     for (size_t i = 0; i < r.size(); ++i) {
       const int32_t o = int32_t((uint32_t(uint16_t(int16_t(r.rows[i]))) << 16) | uint16_t(int16_t(r.cols[i])));
       const float wf = float(r.w[i]);
-      int32_t wbits;
-      std::memcpy(&wbits, &wf, sizeof(wbits));
       offs.push_back(o);
       w.push_back(wf);
-      sw.push_back(make_int2(o, wbits));
-      lw.push_back(make_int2(r.rows[i] * lin_pitch + r.cols[i], wbits));
       wsum += double(wf);
     }
     d.wsum = float(wsum);
@@ -169,12 +162,8 @@ struct DevLevel {
   }
   void upload() {
     retire(d_desc);
-    retire(d_offs);
-    retire(d_runs);
-    retire(d_runs_end);
     retire(d_w);
     retire(d_sw);
-    retire(d_lw);
     retire(d_run4);
     std::vector<int4> run4(runs.size());
     for (const PatchDesc& p : desc) {
@@ -187,27 +176,19 @@ struct DevLevel {
     }
     d_run4.upload(run4, nullptr);
     d_desc.upload(desc, nullptr);
-    d_sw.upload(sw, nullptr);
-    d_lw.upload(lw, nullptr);
+    DevBuf<int32_t> d_offs;
     d_offs.upload(offs, nullptr);
-    d_runs.upload(runs, nullptr);
-    d_runs_end.upload(runs_end, nullptr);
     d_w.upload(w, nullptr);
+    d_sw.reserve(offs.size());
+    check(launch_interleave(d_offs.p, d_w.p, d_sw.p, offs.size(), nullptr), "model upload");
     check(cudaDeviceSynchronize(), "model upload");
   }
   LevelView view() const {
     LevelView v;
     v.patches = d_desc.p;
-    v.offs = d_offs.p;
     v.w = d_w.p;
     v.sw = d_sw.p;
-    v.lw = d_lw.p;
-    v.lin_pitch = lin_pitch;
-    v.lin_rows = lin_rows;
-    v.runs = d_runs.p;
-    v.runs_end = d_runs_end.p;
     v.run4 = d_run4.p;
-    v.npatches = int32_t(desc.size());
     return v;
   }
 };
@@ -282,23 +263,19 @@ void finish_model(mvg_ncc_model_s& m) {
   }
   check(cudaGetDevice(&m.device), "cudaGetDevice");
   std::vector<std::unique_ptr<DevLevel>> levels;
-  std::vector<int32_t> pitch;
   for (const ModelLevel& L : m.host.levels) {
     auto d = std::make_unique<DevLevel>();
     d->set_geometry(L.width, L.height);
-    pitch.push_back(d->lin_pitch);
     levels.push_back(std::move(d));
   }
   std::vector<LevelTables> t;
-  build_tables_device(m.host, pitch, t, nullptr);
+  build_tables_device(m.host, t, nullptr);
   for (size_t l = 0; l < levels.size(); ++l) {
     DevLevel& d = *levels[l];
     d.desc = std::move(t[l].desc);
     d.angles = std::move(t[l].angles);
     d.offs = std::move(t[l].offs);
     d.w = std::move(t[l].w);
-    d.sw = std::move(t[l].sw);
-    d.lw = std::move(t[l].lw);
     d.runs = std::move(t[l].runs);
     d.runs_end = std::move(t[l].runs_end);
     d.model_patches = d.desc.size();
@@ -2618,8 +2595,6 @@ int32_t mvg_ncc_model_tables_digest(mvg_ncc_model model_id, uint64_t* digest) {
       const size_t nr = np ? size_t(L->desc[np - 1].run_off + L->desc[np - 1].nruns) : 0;
       mix(L->offs.data(), ns * sizeof(int32_t));
       mix(L->w.data(), ns * sizeof(float));
-      mix(L->sw.data(), ns * sizeof(int2));
-      mix(L->lw.data(), ns * sizeof(int2));
       mix(L->runs.data(), nr * sizeof(int32_t));
       mix(L->runs_end.data(), nr * sizeof(int32_t));
     }

@@ -32,7 +32,6 @@ struct LevelData {
   const uint8_t* mask;
   int w, h;
   double orow, ocol;
-  int lin_pitch;
 };
 
 struct RasterJob {
@@ -254,17 +253,13 @@ __global__ void __launch_bounds__(32) raster_moments_kernel(const RasterJob* job
 }
 
 // Packs one raster's samples into the level tables (the layout DevLevel
-// builds on the host): packed int16 (row, column), float weight,
-// interleaved {offset, weight bits} and {row * lin_pitch + column, weight
-// bits}, and the row runs (packed row and begin; end).
-__global__ void __launch_bounds__(kBuildThreads) raster_tables_kernel(const RasterJob* jobs, const LevelData* levels,
-                                                                      const int* samples, const int2* rc,
-                                                                      const double* v, int32_t* offs, float* w,
-                                                                      int2* sw, int2* lw, int32_t* runs,
-                                                                      int32_t* runs_end) {
+// builds on the host): packed int16 (row, column), float weight, and the row
+// runs (packed row and begin; end).
+__global__ void __launch_bounds__(kBuildThreads) raster_tables_kernel(const RasterJob* jobs, const int* samples,
+                                                                      const int2* rc, const double* v, int32_t* offs,
+                                                                      float* w, int32_t* runs, int32_t* runs_end) {
   const RasterJob job = jobs[blockIdx.x];
   const int n = samples[blockIdx.x];
-  const int pitch = levels[job.level].lin_pitch;
   const int2* p = rc + job.sample_off;
   int run_base = job.run_off;
   for (int t0 = 0; t0 < n; t0 += blockDim.x) {
@@ -280,11 +275,8 @@ __global__ void __launch_bounds__(kBuildThreads) raster_tables_kernel(const Rast
     if (i < n) {
       const long long g = job.table_off + i;
       const int32_t o = int32_t((uint32_t(uint16_t(int16_t(q.x))) << 16) | uint16_t(int16_t(q.y)));
-      const float wf = __double2float_rn(v[job.sample_off + i]);
       offs[g] = o;
-      w[g] = wf;
-      sw[g] = make_int2(o, __float_as_int(wf));
-      lw[g] = make_int2(q.x * pitch + q.y, __float_as_int(wf));
+      w[g] = __double2float_rn(v[job.sample_off + i]);
       const int run = run_base + incl - 1;
       if (starts) runs[run] = o;
       const bool last = i + 1 == n || p[i + 1].x != q.x || p[i + 1].y != q.y + 1;
@@ -335,8 +327,7 @@ constexpr long long kChunkPositions = 16ll << 20;  // dense positions per chunk 
 
 }  // namespace
 
-void build_tables_device(const HostModel& m, const std::vector<int32_t>& lin_pitch, std::vector<LevelTables>& out,
-                         cudaStream_t s) {
+void build_tables_device(const HostModel& m, std::vector<LevelTables>& out, cudaStream_t s) {
   const size_t nl = m.levels.size();
   out.assign(nl, LevelTables{});
   // level rasters on the device
@@ -350,7 +341,7 @@ void build_tables_device(const HostModel& m, const std::vector<int32_t>& lin_pit
     const size_t px = L.width * L.height;
     cuda_ok(cudaMemcpyAsync(gray[l]->get(px), L.gray.data(), px * sizeof(double), cudaMemcpyHostToDevice, s), "gray");
     cuda_ok(cudaMemcpyAsync(mask[l]->get(px), L.mask.data(), px, cudaMemcpyHostToDevice, s), "mask");
-    ld[l] = LevelData{gray[l]->p, mask[l]->p, int(L.width), int(L.height), L.orow, L.ocol, lin_pitch[l]};
+    ld[l] = LevelData{gray[l]->p, mask[l]->p, int(L.width), int(L.height), L.orow, L.ocol};
   }
   Buf<LevelData> d_levels;
   cuda_ok(cudaMemcpyAsync(d_levels.get(nl), ld.data(), nl * sizeof(LevelData), cudaMemcpyHostToDevice, s), "levels");
@@ -392,7 +383,6 @@ void build_tables_device(const HostModel& m, const std::vector<int32_t>& lin_pit
   Buf<int4> d_bounds;
   Buf<int32_t> d_offs, d_runsv, d_runs_end;
   Buf<float> d_w;
-  Buf<int2> d_sw, d_lw;
   size_t total = 0;  // samples of the rasters accepted so far (budget)
   for (size_t first = 0; first < all.size();) {
     // one chunk of consecutive rasters
@@ -450,9 +440,9 @@ void build_tables_device(const HostModel& m, const std::vector<int32_t>& lin_pit
       if (size_t(ns[size_t(k)]) > m.sample_budget - total) raise(kLimitExceeded, "model raster budget exceeded");
       total += size_t(ns[size_t(k)]);
     }
-    raster_tables_kernel<<<nj, kBuildThreads, 0, s>>>(
-        d_jobs.p, d_levels.p, d_samples.p, d_rc.p, d_v.p, d_offs.get(size_t(samples)), d_w.get(size_t(samples)),
-        d_sw.get(size_t(samples)), d_lw.get(size_t(samples)), d_runsv.get(size_t(runs)), d_runs_end.get(size_t(runs)));
+    raster_tables_kernel<<<nj, kBuildThreads, 0, s>>>(d_jobs.p, d_samples.p, d_rc.p, d_v.p,
+                                                      d_offs.get(size_t(samples)), d_w.get(size_t(samples)),
+                                                      d_runsv.get(size_t(runs)), d_runs_end.get(size_t(runs)));
     cuda_ok(cudaGetLastError(), "raster tables");
     // level tables on the host, raster by raster (a chunk may span levels)
     for (int k = 0; k < nj;) {
@@ -483,8 +473,6 @@ void build_tables_device(const HostModel& m, const std::vector<int32_t>& lin_pit
       }
       to_host(T.offs, d_offs.p + s0, size_t(s1 - s0), s);
       to_host(T.w, d_w.p + s0, size_t(s1 - s0), s);
-      to_host(T.sw, d_sw.p + s0, size_t(s1 - s0), s);
-      to_host(T.lw, d_lw.p + s0, size_t(s1 - s0), s);
       to_host(T.runs, d_runsv.p + r0, size_t(r1 - r0), s);
       to_host(T.runs_end, d_runs_end.p + r0, size_t(r1 - r0), s);
       k = e;

@@ -2673,7 +2673,17 @@ __global__ void domain_cols_kernel(int w, int h, int32_t* count) {
   }
 }
 
+__global__ void interleave_kernel(const int32_t* offs, const float* w, int2* sw, size_t n) {
+  const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i < n) sw[i] = make_int2(offs[i], __float_as_int(w[i]));
+}
+
 // --------------------------------------------------------------- launchers
+cudaError_t launch_interleave(const int32_t* offs, const float* w, int2* sw, size_t n, cudaStream_t s) {
+  if (n) interleave_kernel<<<unsigned((n + 255) / 256), 256, 0, s>>>(offs, w, sw, n);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_domain_count(const uint8_t* mask, int w, int h, int32_t* count, cudaStream_t s) {
   domain_rows_kernel<<<(h + 127) / 128, 128, 0, s>>>(mask, w, h, count);
   domain_cols_kernel<<<(w + 1 + 255) / 256, 256, 0, s>>>(w, h, count);

@@ -128,6 +128,9 @@ struct TrackArgs {
   DomainView dom;
 };
 
+// sw[i] = {offs[i], float bits of w[i]}
+cudaError_t launch_interleave(const int32_t* offs, const float* w, int2* sw, size_t n, cudaStream_t s);
+
 // Raises a kernel's dynamic shared-memory limit on the current device to at
 // least `bytes` (never lowers it; safe from several host threads).
 cudaError_t reserve_dynamic_smem(const void* kernel, size_t bytes);

@@ -51,16 +51,9 @@ struct PatchDesc {
 // Device view of one model level (its patches and their samples).
 struct LevelView {
   const PatchDesc* patches;
-  const int32_t* offs;          // packed (row << 16) | (col & 0xffff), int16 each
   const float* w;               // sample weights (float of the FP64 model weight)
-  const int2* sw;               // interleaved {offs, float bits of w} per sample
-  const int2* lw;               // interleaved {row * lin_pitch + col, float bits of w} per sample
-  int32_t lin_pitch;            // row pitch of lw offsets (= 5 mod 32)
-  int32_t lin_rows;             // rows of a window that holds any 5x5 placement set
-  const int32_t* runs;          // packed row(16) | begin; end in runs_end
-  const int32_t* runs_end;
+  const int2* sw;               // per sample {(row << 16) | (col & 0xffff), float bits of w}
   const int4* run4;             // {row, begin, end, the patch's samples before the run}
-  int32_t npatches;
 };
 
 // Unrotated full-resolution template used for continuous scoring and the
