@@ -498,6 +498,7 @@ __device__ __forceinline__ bool track_valid(const TrackArgs& a, const PatchDesc&
 // runs of successive rows begin and end within a few columns of one
 // another): a step's 25 prefix entries lie in one or two cache lines instead
 // of five.  The sums are exact integers, so their order is free.
+template <int U>  // runs in flight with int64 prefixes
 __device__ __forceinline__ void lane_moments(const LevelImage& lev, int pitch, int r, int c,
                                              const int4* __restrict__ runs, int nruns, int dr, long long& s1,
                                              long long& s2) {
@@ -542,15 +543,22 @@ __device__ __forceinline__ void lane_moments(const LevelImage& lev, int pitch, i
   }
   const longlong2* __restrict__ P = lev.prefix;
   int j = 0;
-  for (; j + 1 < nruns; j += 2) {
-    const int4 q0 = next(), q1 = next();
-    const size_t b0 = size_t(r + q0.x) * pitch + c, b1 = size_t(r + q1.x) * pitch + c;
-    const longlong2 h0 = P[b0 + q0.z + 1], l0 = P[b0 + q0.y];
-    const longlong2 h1 = P[b1 + q1.z + 1], l1 = P[b1 + q1.y];
-    s1 += (h0.x - l0.x) + (h1.x - l1.x);
-    s2 += (h0.y - l0.y) + (h1.y - l1.y);
+  for (; j + U - 1 < nruns; j += U) {
+    longlong2 hi[U], lo[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int4 q = next();
+      const size_t base = size_t(r + q.x) * pitch + c;
+      hi[u] = P[base + q.z + 1];
+      lo[u] = P[base + q.y];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      s1 += hi[u].x - lo[u].x;
+      s2 += hi[u].y - lo[u].y;
+    }
   }
-  if (j < nruns) {
+  for (; j < nruns; ++j) {
     const int4 q = next();
     const size_t base = size_t(r + q.x) * pitch + c;
     const longlong2 hi = P[base + q.z + 1], lo = P[base + q.y];
@@ -602,6 +610,22 @@ __device__ __forceinline__ int2 runs_meeting(const int4* __restrict__ runs, int 
   return make_int2(first, last);
 }
 
+// Two FP32 values in a 64-bit register pair, and acc += a * b on both.
+using F32x2 = unsigned long long;
+__device__ __forceinline__ F32x2 twice(float x) {
+  F32x2 r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float2 halves(F32x2 x) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(x));
+  return r;
+}
+__device__ __forceinline__ void fma_both(F32x2& acc, F32x2 a, F32x2 b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+
 // sum w (S - centre) of one patch at the 25 positions from a window in shared
 // memory (values minus its centre value); lane p < 25 returns position p's.
 // Position (0, 0) puts the patch's row y and column x on window row
@@ -610,16 +634,19 @@ __device__ __forceinline__ int2 runs_meeting(const int4* __restrict__ runs, int 
 // columns each, and the eight groups of four lanes share the runs that meet
 // the strip, so a strip costs about an eighth of its rows.  A lane walks down
 // its rows with the 5 x 8 values under its four samples in registers: per
-// row two 16-byte reads and four weights feed 100 FMAs.
+// row two 16-byte reads and four weights feed 100 multiply-adds.  The values
+// sit in pairs of columns, so that 80 of them are 40 two-wide instructions
+// (the kernel is bound by the instructions it issues); an even and an odd
+// sample column pair the placements differently and have their own sums.
 __device__ __forceinline__ float staged_dots(const float* win, int pitch, const LevelView& view, const PatchDesc& pd,
                                              int rshift, int cshift, int strip0, int step) {
   const int lane = threadIdx.x & 31, group = lane >> 2;
   const int4* __restrict__ runs = view.run4 + pd.run_off;
   const float* __restrict__ weights = view.w + pd.sample_off;
   const int xlast = (pd.cmax + cshift) & ~3;  // window columns of the last samples
-  float acc[25];
-#pragma unroll
-  for (int i = 0; i < 25; ++i) acc[i] = 0.f;
+  // sums by placement row: even sample columns dc (0, 1), (2, 3), 4; odd ones 0, (1, 2), (3, 4)
+  F32x2 e01[5] = {}, e23[5] = {}, o12[5] = {}, o34[5] = {};
+  float e4[5] = {}, o0[5] = {};
   for (int base = ((pd.cmin + cshift) & ~3) + 16 * strip0; base <= xlast; base += 16 * step) {
     const int2 span = runs_meeting(runs, pd.nruns, base - cshift, base + 15 - cshift);
     if (span.y < 0) continue;
@@ -628,46 +655,68 @@ __device__ __forceinline__ float staged_dots(const float* win, int pitch, const 
     const int X = min(base + 4 * (lane & 3), xlast);  // past the patch: repeats its last columns, no weights
     const int x = base + 4 * (lane & 3) - cshift;     // first sample column
     const float* col = win + X;
-    float v[5][8];  // window row y + i in v[(i + phase) % 5]
+    F32x2 v[5][4];  // window row y + i in v[(i + phase) % 5], columns in pairs
+    auto load = [&](F32x2 (&r)[4], const float* at) {
+      const ulonglong2 lo = *reinterpret_cast<const ulonglong2*>(at), hi = *reinterpret_cast<const ulonglong2*>(at + 4);
+      r[0] = lo.x, r[1] = lo.y, r[2] = hi.x, r[3] = hi.y;
+    };
+    // the next run and its weights are loaded one row ahead of their use
+    auto run_at = [&](int j) { return __ldg(runs + min(j, pd.nruns - 1)); };
+    auto weights_of = [&](const int4& q, bool live, float (&w)[4]) {
+      const int u = x - q.y;
+      const unsigned len = unsigned(q.z - q.y);
+      const float* wp = weights + q.w + u;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) w[e] = live && unsigned(u + e) <= len ? __ldg(wp + e) : 0.f;
+    };
+    int4 next = run_at(j0);
+    float wn[4];
+    weights_of(next, j0 <= j1, wn);
+    int4 after = run_at(j0 + 1);
     int ynext = INT32_MIN;
     for (int it = 0; it < per; it += 5) {
 #pragma unroll
       for (int phase = 0; phase < 5; ++phase) {
         const int j = j0 + it + phase;
         if (it + phase < per && j <= j1) {
-          const int4 q = __ldg(runs + j);
-          const float* row = col + (q.x + rshift) * pitch;
-          if (q.x != ynext) {
+          const float* row = col + (next.x + rshift) * pitch;
+          if (next.x != ynext) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const float4 lo = *reinterpret_cast<const float4*>(row + i * pitch);
-              const float4 hi = *reinterpret_cast<const float4*>(row + i * pitch + 4);
-              float(&r)[8] = v[(phase + i) % 5];
-              r[0] = lo.x, r[1] = lo.y, r[2] = lo.z, r[3] = lo.w, r[4] = hi.x, r[5] = hi.y, r[6] = hi.z, r[7] = hi.w;
+            for (int i = 0; i < 4; ++i) load(v[(phase + i) % 5], row + i * pitch);
+          }
+          load(v[(phase + 4) % 5], row + 4 * pitch);
+          ynext = next.x + 1;
+          const float w[4] = {wn[0], wn[1], wn[2], wn[3]};
+          next = after;
+          weights_of(next, j + 1 <= j1, wn);
+          after = run_at(j + 2);
+          const F32x2 ww[4] = {twice(w[0]), twice(w[1]), twice(w[2]), twice(w[3])};
+#pragma unroll
+          for (int i = 0; i < 5; ++i) {
+            const F32x2(&r)[4] = v[(phase + i) % 5];
+#pragma unroll
+            for (int e = 0; e < 4; e += 2) {
+              fma_both(e01[i], ww[e], r[e / 2]);
+              fma_both(e23[i], ww[e], r[e / 2 + 1]);
+              e4[i] = fmaf(w[e], halves(r[e / 2 + 2 < 4 ? e / 2 + 2 : 3]).x, e4[i]);
+              o0[i] = fmaf(w[e + 1], halves(r[e / 2]).y, o0[i]);
+              fma_both(o12[i], ww[e + 1], r[e / 2 + 1]);
+              fma_both(o34[i], ww[e + 1], r[e / 2 + 2 < 4 ? e / 2 + 2 : 3]);
             }
           }
-          {
-            const float4 lo = *reinterpret_cast<const float4*>(row + 4 * pitch);
-            const float4 hi = *reinterpret_cast<const float4*>(row + 4 * pitch + 4);
-            float(&r)[8] = v[(phase + 4) % 5];
-            r[0] = lo.x, r[1] = lo.y, r[2] = lo.z, r[3] = lo.w, r[4] = hi.x, r[5] = hi.y, r[6] = hi.z, r[7] = hi.w;
-          }
-          ynext = q.x + 1;
-          const unsigned len = unsigned(q.z - q.y);
-          const int u = x - q.y;
-          const float* wp = weights + q.w + u;
-          float w[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) w[e] = unsigned(u + e) <= len ? __ldg(wp + e) : 0.f;
-#pragma unroll
-          for (int i = 0; i < 5; ++i)
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-#pragma unroll
-              for (int d = 0; d < 5; ++d) acc[5 * i + d] = fmaf(w[e], v[(phase + i) % 5][e + d], acc[5 * i + d]);
         }
       }
     }
+  }
+  float acc[25];
+#pragma unroll
+  for (int i = 0; i < 5; ++i) {
+    const float2 a = halves(e01[i]), b = halves(e23[i]), c = halves(o12[i]), d = halves(o34[i]);
+    acc[5 * i] = a.x + o0[i];
+    acc[5 * i + 1] = a.y + c.x;
+    acc[5 * i + 2] = b.x + c.y;
+    acc[5 * i + 3] = b.y + d.x;
+    acc[5 * i + 4] = e4[i] + d.y;
   }
   return lane_total25(acc);
 }
@@ -810,7 +859,7 @@ __global__ void __launch_bounds__(32 * kTrackWarps, 8) track_warp_kernel(const _
       const float dot = left >> k & 1 ? s_dot[min(1, __popc(left & ((1u << k) - 1)))][lane]
                                       : track_tc_dot(a, pd, src, i, k, lane, r, c);
       long long s1, s2;
-      lane_moments(a.lev, a.lev.w + 1, r, c, a.view.run4 + pd.run_off, pd.nruns, dr, s1, s2);
+      lane_moments<2>(a.lev, a.lev.w + 1, r, c, a.view.run4 + pd.run_off, pd.nruns, dr, s1, s2);
       const float sc = window_score(dot, s1, s2, pd.n, a.absolute);
       if (better(sc, k * 25 + lane, best, border)) {
         best = sc;
@@ -846,13 +895,15 @@ __global__ void __launch_bounds__(32 * kTrackWarps, 8) track_warp_kernel(const _
 // Other levels: one block per candidate.  The union window of the patches
 // the block correlates is staged in shared memory, centred on one of its
 // pixels (exact small integers in float; zero outside the level); the warps
-// take (patch, strip group) tasks and (patch, moments) tasks, and then the
-// items are scored.  Windows larger than shared memory read the level.
-// Bound by the instructions of staged_dots (FP32 pipes) and the latency of
-// the small patches' prologues.  uint16 lists, two steps at 2048^2 with a
-// 128^2 template (3.1 G multiply-adds): 1.98 -> 1.09 ms; three at 4096^2 with
-// 256^2 (21 G): 40 -> 5.8 ms (one shared-memory read and one weight read per
-// multiply-add before).
+// take (patch, strip group) and (patch, run group) tasks, and then the items
+// are scored.  Windows larger than shared memory read the level.  Bound by
+// the latency of a candidate's phases with the 16 warps per SM that the
+// register tiles leave (set-up and staging a quarter of them, dots and
+// moments 60 %).  uint16 lists, two steps at 2048^2 with a 128^2 template
+// (3.1 G multiply-adds): 1.98 -> 0.92 ms; three at 4096^2 with 256^2 (21 G):
+// 40 -> 5.2 ms (one shared-memory read and one weight read per multiply-add,
+// and a 256-thread block per possible candidate, before; 1.09 and 5.8 with
+// 256-thread blocks here).
 __global__ void __launch_bounds__(512) track_block_kernel(TrackArgs a) {
   extern __shared__ float smem[];
   __shared__ int s_row[kTrackMaxSel], s_col[kTrackMaxSel];
@@ -875,6 +926,7 @@ __global__ void __launch_bounds__(512) track_block_kernel(TrackArgs a) {
     const TrackCentre t = track_centre(a, cd);
     if (warp == 0) {
       int wr0 = INT32_MAX, wc0 = INT32_MAX, wr1 = INT32_MIN, wc1 = INT32_MIN;
+      unsigned samples = 0;
       for (int k = lane; k < n; k += 32) {
         const PatchDesc pd = a.view.patches[a.plist[a.sel_idx[sel0 + k]]];
         const int row = track_row(a, t, pd), col = track_col(a, t, pd);
@@ -883,6 +935,7 @@ __global__ void __launch_bounds__(512) track_block_kernel(TrackArgs a) {
         const bool istc = tc && pd.lattice && k < kTcMaxP;
         s_istc[k] = istc;
         if (!istc) {
+          samples += unsigned(pd.n);
           wr0 = min(wr0, row - 2 + pd.rmin);
           wr1 = max(wr1, row + 2 + pd.rmax);
           wc0 = min(wc0, col - 2 + pd.cmin);
@@ -893,7 +946,9 @@ __global__ void __launch_bounds__(512) track_block_kernel(TrackArgs a) {
       wc0 = __reduce_min_sync(0xffffffffu, wc0);
       wr1 = __reduce_max_sync(0xffffffffu, wr1);
       wc1 = __reduce_max_sync(0xffffffffu, wc1);
+      samples = __reduce_add_sync(0xffffffffu, samples);
       if (lane == 0) {
+        if (samples) atomicAdd(&a.state->track_macs, 25ull * samples);
         s_bound[0] = wr0;
         s_bound[1] = wr1;
         s_bound[2] = wc0;
@@ -910,36 +965,49 @@ __global__ void __launch_bounds__(512) track_block_kernel(TrackArgs a) {
       const int cr = min(max(wr0 + wh / 2, 0), a.lev.h - 1), cc = min(max(wc0 + ww / 2, 0), a.lev.w - 1);
       centre = a.lev.v[size_t(cr) * a.lev.w + cc];
     }
+    for (int t = threadIdx.x; t < n * 32; t += blockDim.x) s_mom[t] = s_mom[a.sel_max * 32 + t] = 0;
     if (staged) {
-      // one warp per row, consecutive columns
-      for (int rr = warp; rr < wh; rr += nwarps) {
-        const int r = wr0 + rr;
-        const bool in = r >= 0 && r < a.lev.h;
-        const float* row = a.lev.v + size_t(in ? r : 0) * a.lev.w + wc0;
-        float* dst = win + rr * a.win_pitch;
-        for (int x = lane; x < min(ww + 4, a.win_pitch); x += 32)
-          dst[x] = in && wc0 + x >= 0 && wc0 + x < a.lev.w ? row[x] - centre : 0.f;
-      }
+      // a warp per row, consecutive columns, four rows in flight
+      const int cols = min(ww + 4, a.win_pitch);
+      for (int r0 = warp; r0 < wh; r0 += 4 * nwarps)
+        for (int x = lane; x < cols; x += 32) {
+          const bool in_x = wc0 + x >= 0 && wc0 + x < a.lev.w;
+          float v[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int r = wr0 + r0 + u * nwarps;
+            v[u] = in_x && r >= 0 && r < a.lev.h ? a.lev.v[size_t(r) * a.lev.w + wc0 + x] - centre : 0.f;
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (r0 + u * nwarps < wh) win[(r0 + u * nwarps) * a.win_pitch + x] = v[u];
+        }
     }
     __syncthreads();
-    for (int task = warp; task < n * (kTrackParts + 1); task += nwarps) {
+    // (patch, strip group) and (patch, run group) tasks; the moments' run
+    // groups keep their loads' latency off the block's critical path
+    constexpr int parts = kTrackParts;
+    for (int task = warp; task < n * 2 * kTrackParts; task += nwarps) {
       const int k = task % n, part = task / n;
       const int j = a.sel_idx[sel0 + k];
       const PatchDesc pd = a.view.patches[a.plist[j]];
-      if (part == kTrackParts) {
+      if (part >= parts) {
         const int dr = lane / 5, dc = lane - 5 * dr;
         const int r = s_row[k] + dr - 2, c = s_col[k] + dc - 2;
-        long long s1 = 0, s2 = 0;
-        if (lane < 25 && track_valid(a, pd, a.ranges[j], r, c))
-          lane_moments(a.lev, a.lev.w + 1, r, c, a.view.run4 + pd.run_off, pd.nruns, dr, s1, s2);
-        s_mom[k * 32 + lane] = s1;
-        s_mom[(a.sel_max + k) * 32 + lane] = s2;
+        const int per = (pd.nruns + kTrackParts - 1) / kTrackParts, first = (part - parts) * per;
+        const int count = min(per, pd.nruns - first);
+        if (count > 0 && lane < 25 && track_valid(a, pd, a.ranges[j], r, c)) {
+          long long s1 = 0, s2 = 0;
+          lane_moments<4>(a.lev, a.lev.w + 1, r, c, a.view.run4 + pd.run_off + first, count, dr, s1, s2);
+          atomicAdd(reinterpret_cast<unsigned long long*>(s_mom + k * 32 + lane), (unsigned long long)s1);
+          atomicAdd(reinterpret_cast<unsigned long long*>(s_mom + (a.sel_max + k) * 32 + lane), (unsigned long long)s2);
+        }
       } else if (!s_istc[k]) {
         const int rs = s_row[k] - 2 - wr0, cs = s_col[k] - 2 - wc0;
         s_dot[(k * kTrackParts + part) * 32 + lane] =
-            staged ? staged_dots(win, a.win_pitch, a.view, pd, rs, cs, part, kTrackParts)
+            staged ? staged_dots(win, a.win_pitch, a.view, pd, rs, cs, part, parts)
                    : level_dots(LevelWindow{a.lev.v, a.lev.w, a.lev.h, wr0, wc0, centre}, a.view, pd, rs, cs, part,
-                                kTrackParts);
+                                parts);
       }
     }
     __syncthreads();
@@ -956,7 +1024,7 @@ __global__ void __launch_bounds__(512) track_block_kernel(TrackArgs a) {
         dot = track_tc_dot(a, pd, src, i, k, pos, r, c);
       } else {
         dot = 0.f;
-        for (int q = 0; q < kTrackParts; ++q) dot += s_dot[(k * kTrackParts + q) * 32 + pos];
+        for (int q = 0; q < parts; ++q) dot += s_dot[(k * kTrackParts + q) * 32 + pos];
         // sum w (S - S0) = sum w (S - centre) - (S0 - centre) sum w
         const int2 f0 = __ldg(a.view.sw + pd.sample_off);
         const float x0 = a.lev.v[size_t(r + off_row(f0.x)) * a.lev.w + c + off_col(f0.x)] - centre;
@@ -982,15 +1050,11 @@ __global__ void __launch_bounds__(512) track_block_kernel(TrackArgs a) {
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-      unsigned long long macs = 0;
       for (int w = 0; w < nwarps; ++w)
         if (better(s_wbest[w], s_word[w], best, border)) {
           best = s_wbest[w];
           border = s_word[w];
         }
-      for (int k = 0; k < n; ++k)
-        if (!s_istc[k]) macs += 25ull * (unsigned long long)a.view.patches[a.plist[a.sel_idx[sel0 + k]]].n;
-      if (macs) atomicAdd(&a.state->track_macs, macs);
       track_write(a, i, cd, best, border, t, sel0);
     }
     __syncthreads();
@@ -2767,8 +2831,11 @@ cudaError_t launch_track(const TrackArgs& a, int max_candidates, cudaStream_t s,
   }
   smem += tables;
   if (const cudaError_t e = reserve_dynamic_smem(reinterpret_cast<const void*>(track_block_kernel), smem)) return e;
-  // a window that leaves room for one block per SM gets 16 warps, others 8
-  const int threads = smem > 100 * 1024 ? 512 : 256;
+  // 128 registers a thread leave an SM 16 warps: in as many blocks as the
+  // window lets in, so that their phases overlap (four blocks of 128 threads
+  // 0.92, two of 256 1.09 ms at 2048^2; one of 256 7.0, of 512 5.8 ms where
+  // the window fills the SM)
+  const int threads = smem > 100 * 1024 ? 512 : smem > 50 * 1024 ? 256 : 128;
   track_block_kernel<<<std::min(max_candidates, 16 * sms), threads, smem, s>>>(b);
   return cudaGetLastError();
 }
