@@ -1299,11 +1299,13 @@ FindOutput run_find(mvg_ncc_model_s& m, const void* pixels, int type, int64_t W,
   // staged tracking windows, and the patches off the lattice (never on the tensor cores)
   int track_window[kMaxLevels] = {};
   std::vector<std::vector<uint8_t>> off_lattice(level_count);
+  std::vector<std::vector<int32_t>> patch_samples(level_count);
   for (size_t li = 0; li < level_count; ++li) {
     track_window[li] = m.levels[li]->lin_rows;
     for (int32_t p : plan[li].plist) {
       const PatchDesc& d = m.levels[li]->desc[size_t(p)];
       off_lattice[li].push_back(d.orow != 0 || d.ocol != 0);
+      patch_samples[li].push_back(d.n);
     }
   }
   // longest run of any patch per level (bounds a run's moment sums)
@@ -1529,6 +1531,7 @@ FindOutput run_find(mvg_ncc_model_s& m, const void* pixels, int type, int64_t W,
     if (type == 1) check(launch_level_range(lev[0], st, s), "level range");
   }
   const size_t first_target = std::max(finest, size_t(opt.subpixel ? 1 : 0));
+  PrefixArgs prefix{};
   for (size_t l = 0; l < level_count; ++l) {
     const bool need = l == top || (l + 1 <= top && l >= first_target);
     if (!need) continue;
@@ -1538,8 +1541,11 @@ FindOutput run_find(mvg_ncc_model_s& m, const void* pixels, int type, int64_t W,
     const double maxv = (type == 1 ? 65535.0 : 255.0) * std::ldexp(1., int(2 * l));
     lev[l].prefix32 =
         double(max_run[l]) * maxv * maxv < 4294967296.0 ? reinterpret_cast<uint2*>(ws.lev_p[l].p) : nullptr;
+    prefix.lev[prefix.n++] = lev[l];
+  }
+  {
     Span sp(kStPrefix, s);
-    check(launch_prefix(lev[l], s), "prefix");
+    check(launch_prefix(prefix, s), "prefix");
   }
 
   // coarse scan + NMS
@@ -1710,6 +1716,11 @@ FindOutput run_find(mvg_ncc_model_s& m, const void* pixels, int type, int64_t W,
       ta.step = std::ldexp(1., int(t));
       ta.offset = (ta.step - 1) * .5;
       ta.exact32 = exact32;
+      ta.crop_row32 = float(crop_row);
+      ta.crop_col32 = float(crop_col);
+      ta.step32 = float(ta.step);
+      ta.offset32 = float(ta.offset);
+      ta.inv_step32 = float(1.0 / ta.step);
       ta.absolute = hm.params.ignore_polarity;
       ta.tc_dots = nullptr;
       ta.tc_group_of_src = nullptr;
@@ -1717,6 +1728,15 @@ FindOutput run_find(mvg_ncc_model_s& m, const void* pixels, int type, int64_t W,
       ta.dom = dv;
       ta.win_rows = track_window[t];
       ta.win_pitch = ((track_window[t] + 3) & ~3) + 4;
+      {
+        // sums of lane_moments_narrow: sum S and four runs' sum S^2 below
+        // 2^32, the variance numerator below 2^62
+        double samples = 0;
+        for (int32_t c : patch_samples[t]) samples = std::max(samples, double(c));
+        const double maxv = (type == 1 ? 65535.0 : 255.0) * std::ldexp(1., int(2 * t));
+        ta.narrow = lev[t].prefix32 && 4.0 * max_run[t] * maxv * maxv < 4294967296.0 &&
+                    samples * maxv < 4294967296.0 && samples * samples * maxv * maxv < 4.6e18;
+      }
       ta.sel_max = 1;
       ta.warp_lists = tc[t] != nullptr;
       for (size_t src = 0; src + 1 < plan[t].sel_off.size(); ++src) {

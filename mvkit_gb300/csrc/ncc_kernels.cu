@@ -125,6 +125,15 @@ __device__ __forceinline__ float window_score(float dot, long long s1, long long
   return absolute ? fabsf(s) : s;
 }
 
+// The same where the variance numerator stays below 2^62.
+__device__ __forceinline__ float window_score_narrow(float dot, uint32_t s1, unsigned long long s2, int n, int absolute) {
+  const long long v = (long long)(s2 * (unsigned long long)n) - (long long)((unsigned long long)s1 * s1);
+  if (v <= 0) return -INFINITY;
+  float s = dot * rsqrtf(__ll2float_rn(v) / float(n));
+  s = fminf(1.f, fmaxf(-1.f, s));
+  return absolute ? fabsf(s) : s;
+}
+
 // Window moments {sum S, sum S^2} of a patch at (r, c) from the level's row
 // prefixes: runs first, first + step, ... (step > 1 splits the runs over
 // threads; the caller adds the parts).
@@ -250,58 +259,64 @@ __global__ void pyramid_kernel(LevelImage src, LevelImage dst, int32_t* error_fl
   dst.v[size_t(r) * dst.w + c] = s;
 }
 
-// row prefix sums {sum S, sum S^2}, one warp per row
-__global__ void prefix_kernel(LevelImage lev) {
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+// Prefixes of one row by a warp: a lane sums four consecutive columns, the
+// lanes' totals are scanned, and the next 128 columns are loaded before this
+// step's scan.  T: uint32 (modulo 2^32, the same stored values) or int64.
+template <class T, class Pair>
+__device__ __forceinline__ void prefix_row(const float* __restrict__ row, int w, Pair* out) {
   const int lane = threadIdx.x & 31;
-  if (warp >= lev.h) return;
-  const float* row = lev.v + size_t(warp) * lev.w;
-  longlong2* out = lev.prefix + size_t(warp) * (lev.w + 1);
-  uint2* out32 = lev.prefix32 ? lev.prefix32 + size_t(warp) * (lev.w + 1) : nullptr;
-  if (lane == 0) {
-    if (out32)
-      out32[0] = make_uint2(0, 0);
-    else
-      out[0] = make_longlong2(0, 0);
-  }
-  if (out32) {
-    // modulo 2^32: the same stored values from 32-bit sums and shuffles
-    uint32_t c1 = 0, c2 = 0;
-    for (int base = 0; base < lev.w; base += 32) {
-      const int c = base + lane;
-      const uint32_t s = c < lev.w ? uint32_t(row[c]) : 0u;
-      uint32_t a = s, b = s * s;
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t ua = __shfl_up_sync(0xffffffffu, a, o);
-        const uint32_t ub = __shfl_up_sync(0xffffffffu, b, o);
-        if (lane >= o) {
-          a += ua;
-          b += ub;
-        }
-      }
-      if (c < lev.w) out32[c + 1] = make_uint2(c1 + a, c2 + b);
-      c1 += __shfl_sync(0xffffffffu, a, 31);
-      c2 += __shfl_sync(0xffffffffu, b, 31);
+  if (lane == 0) out[0] = Pair{0, 0};
+  auto load = [&](int base, float (&v)[4]) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = base + 4 * lane + k < w ? row[base + 4 * lane + k] : 0.f;
+  };
+  float next[4];
+  load(0, next);
+  T c1 = 0, c2 = 0;
+  for (int base = 0; base < w; base += 128) {
+    T a[4], b[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const T s = T(next[k]);
+      a[k] = (k ? a[k - 1] : T(0)) + s;
+      b[k] = (k ? b[k - 1] : T(0)) + s * s;
     }
-    return;
-  }
-  long long c1 = 0, c2 = 0;
-  for (int base = 0; base < lev.w; base += 32) {
-    const int c = base + lane;
-    const long long s = c < lev.w ? (long long)row[c] : 0;
-    long long a = s, b = s * s;
+    load(base + 128, next);
+    T t1 = a[3], t2 = b[3];
+#pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const long long ua = __shfl_up_sync(0xffffffffu, a, o);
-      const long long ub = __shfl_up_sync(0xffffffffu, b, o);
+      const T u1 = __shfl_up_sync(0xffffffffu, t1, o), u2 = __shfl_up_sync(0xffffffffu, t2, o);
       if (lane >= o) {
-        a += ua;
-        b += ub;
+        t1 += u1;
+        t2 += u2;
       }
     }
-    if (c < lev.w) out[c + 1] = make_longlong2(c1 + a, c2 + b);
-    c1 += __shfl_sync(0xffffffffu, a, 31);
-    c2 += __shfl_sync(0xffffffffu, b, 31);
+    const T e1 = c1 + t1 - a[3], e2 = c2 + t2 - b[3];  // before this lane's columns
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int c = base + 4 * lane + k;
+      if (c < w) out[c + 1] = Pair{e1 + a[k], e2 + b[k]};
+    }
+    c1 += __shfl_sync(0xffffffffu, t1, 31);
+    c2 += __shfl_sync(0xffffffffu, t2, 31);
   }
+}
+
+// Row prefix sums {sum S, sum S^2}, one warp per row, the rows of every level
+// of the find in one launch (the widest level first): the levels' chains of
+// row steps run side by side.  Three levels of 2048^2: 0.043 -> 0.010 ms (a launch
+// per level, 32 columns per step before).
+__global__ void prefix_kernel(const __grid_constant__ PrefixArgs a) {
+  int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, l = 0;
+  while (l < a.n && warp >= a.lev[l].h) warp -= a.lev[l++].h;
+  if (l >= a.n) return;
+  const LevelImage& lev = a.lev[l];
+  const float* row = lev.v + size_t(warp) * lev.w;
+  const size_t at = size_t(warp) * (lev.w + 1);
+  if (lev.prefix32)
+    prefix_row<uint32_t>(row, lev.w, lev.prefix32 + at);
+  else
+    prefix_row<long long>(row, lev.w, lev.prefix + at);
 }
 
 // ---------------------------------------------------------------- coarse scan
@@ -470,9 +485,8 @@ struct TrackCentre {
 __device__ __forceinline__ TrackCentre track_centre(const TrackArgs& a, const Cand& cd) {
   TrackCentre t{};
   if (a.exact32) {
-    const float s = float(1.0 / a.step);
-    t.x32r = __fmul_rn(__fsub_rn(__fsub_rn(float(cd.row), float(a.crop_row)), float(a.offset)), s);
-    t.x32c = __fmul_rn(__fsub_rn(__fsub_rn(float(cd.col), float(a.crop_col)), float(a.offset)), s);
+    t.x32r = __fmul_rn(__fsub_rn(__fsub_rn(float(cd.row), a.crop_row32), a.offset32), a.inv_step32);
+    t.x32c = __fmul_rn(__fsub_rn(__fsub_rn(float(cd.col), a.crop_col32), a.offset32), a.inv_step32);
   } else {
     t.xr = dsub(dsub(cd.row, a.crop_row), a.offset) / a.step;
     t.xc = dsub(dsub(cd.col, a.crop_col), a.offset) / a.step;
@@ -522,9 +536,9 @@ __device__ __forceinline__ void lane_moments(const LevelImage& lev, int pitch, i
       uint2 hi[4], lo[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        const size_t base = size_t(r + q[u].x) * pitch + c;
-        hi[u] = P[base + q[u].z + 1];
-        lo[u] = P[base + q[u].y];
+        const uint32_t base = uint32_t(r + q[u].x) * uint32_t(pitch) + uint32_t(c);
+        hi[u] = P[base + uint32_t(q[u].z + 1)];
+        lo[u] = P[base + uint32_t(q[u].y)];
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
@@ -534,8 +548,8 @@ __device__ __forceinline__ void lane_moments(const LevelImage& lev, int pitch, i
     }
     for (; j < nruns; ++j) {
       const int4 q = next();
-      const size_t base = size_t(r + q.x) * pitch + c;
-      const uint2 hi = P[base + q.z + 1], lo = P[base + q.y];
+      const uint32_t base = uint32_t(r + q.x) * uint32_t(pitch) + uint32_t(c);
+      const uint2 hi = P[base + uint32_t(q.z + 1)], lo = P[base + uint32_t(q.y)];
       s1 += (long long)(hi.x - lo.x);
       s2 += (long long)(hi.y - lo.y);
     }
@@ -548,9 +562,9 @@ __device__ __forceinline__ void lane_moments(const LevelImage& lev, int pitch, i
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int4 q = next();
-      const size_t base = size_t(r + q.x) * pitch + c;
-      hi[u] = P[base + q.z + 1];
-      lo[u] = P[base + q.y];
+      const uint32_t base = uint32_t(r + q.x) * uint32_t(pitch) + uint32_t(c);
+      hi[u] = P[base + uint32_t(q.z + 1)];
+      lo[u] = P[base + uint32_t(q.y)];
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -560,10 +574,46 @@ __device__ __forceinline__ void lane_moments(const LevelImage& lev, int pitch, i
   }
   for (; j < nruns; ++j) {
     const int4 q = next();
-    const size_t base = size_t(r + q.x) * pitch + c;
-    const longlong2 hi = P[base + q.z + 1], lo = P[base + q.y];
+    const uint32_t base = uint32_t(r + q.x) * uint32_t(pitch) + uint32_t(c);
+    const longlong2 hi = P[base + uint32_t(q.z + 1)], lo = P[base + uint32_t(q.y)];
     s1 += hi.x - lo.x;
     s2 += hi.y - lo.y;
+  }
+}
+
+// The same with 32-bit sums, where the host found that sum S of a window and
+// sum S^2 of any four runs stay below 2^32 (uint8 levels 1 and 2): the index
+// and sum arithmetic around the loads is what bounds these levels.
+__device__ __forceinline__ void lane_moments_narrow(const LevelImage& lev, int pitch, int r, int c,
+                                                    const int4* __restrict__ runs, int nruns, int dr, uint32_t& s1,
+                                                    unsigned long long& s2) {
+  const uint2* __restrict__ P = lev.prefix32 + (size_t(r) * pitch + c);
+  int at = nruns - dr;
+  while (at < 0) at += nruns;
+  if (at == nruns) at = 0;
+  s1 = 0;
+  s2 = 0;
+  for (int j = 0; j < nruns; j += 4) {
+    uint2 hi[4], lo[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int4 q = __ldg(runs + at);
+      if (j + u < nruns) {
+        if (++at == nruns) at = 0;
+        const int base = q.x * pitch;
+        hi[u] = P[base + q.z + 1];
+        lo[u] = P[base + q.y];
+      } else {
+        hi[u] = lo[u] = make_uint2(0, 0);
+      }
+    }
+    uint32_t four = 0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      s1 += hi[u].x - lo[u].x;
+      four += hi[u].y - lo[u].y;
+    }
+    s2 += four;
   }
 }
 
@@ -769,8 +819,8 @@ __device__ void track_write(const TrackArgs& a, int i, const Cand& cd, float bes
     const PatchDesc pd = a.view.patches[pi];
     const int r = track_row(a, t, pd) + l / 5 - 2, c = track_col(a, t, pd) + l % 5 - 2;
     if (a.exact32) {
-      out.row = double(lattice_pose32(float(a.crop_row), float(a.step), r, float(pd.orow), float(a.offset)));
-      out.col = double(lattice_pose32(float(a.crop_col), float(a.step), c, float(pd.ocol), float(a.offset)));
+      out.row = double(lattice_pose32(a.crop_row32, a.step32, r, pd.orow32, a.offset32));
+      out.col = double(lattice_pose32(a.crop_col32, a.step32, c, pd.ocol32, a.offset32));
     } else {
       out.row = lattice_pose(a.crop_row, a.step, r, pd.orow, a.offset);
       out.col = lattice_pose(a.crop_col, a.step, c, pd.ocol, a.offset);
@@ -797,9 +847,9 @@ __device__ __forceinline__ float track_tc_dot(const TrackArgs& a, const PatchDes
 // the score and the choice.  The few patches the tensor cores left out are
 // correlated first, by the block.  Bound by the instructions around the
 // prefix loads and their latency.  2048^2 u8, 128^2 template, two steps: 0.27
-// -> 0.17 ms; 57,000 candidates of a 48^2 template over a full circle: 1.03 ->
-// 0.60 ms (one 256-thread block per possible candidate before, each step's
-// lanes on five image rows).
+// -> 0.16 ms; 57,000 candidates of a 48^2 template over a full circle: 1.03 ->
+// 0.56 ms (one 256-thread block per possible candidate before, each step's
+// lanes on five image rows; 0.17 and 0.61 with 64-bit sums and indices).
 
 // Dots of patch k of candidate cd, sum w (S - S0), by the whole block, to
 // out[position].  Kept out of line: few candidates need it, and its registers
@@ -825,6 +875,7 @@ __device__ __noinline__ void plain_dots(const TrackArgs& a, const Cand& cd, int 
   __syncthreads();
 }
 
+template <bool Narrow>
 __global__ void __launch_bounds__(32 * kTrackWarps, 8) track_warp_kernel(const __grid_constant__ TrackArgs a) {
   __shared__ float s_part[kTrackWarps][32], s_dot[2][32];
   __shared__ float s_best[kTrackWarps];
@@ -858,9 +909,17 @@ __global__ void __launch_bounds__(32 * kTrackWarps, 8) track_warp_kernel(const _
       if (lane >= 25 || !track_valid(a, pd, a.ranges[j], r, c)) continue;
       const float dot = left >> k & 1 ? s_dot[min(1, __popc(left & ((1u << k) - 1)))][lane]
                                       : track_tc_dot(a, pd, src, i, k, lane, r, c);
-      long long s1, s2;
-      lane_moments<2>(a.lev, a.lev.w + 1, r, c, a.view.run4 + pd.run_off, pd.nruns, dr, s1, s2);
-      const float sc = window_score(dot, s1, s2, pd.n, a.absolute);
+      float sc;
+      if (Narrow) {
+        uint32_t s1;
+        unsigned long long s2;
+        lane_moments_narrow(a.lev, a.lev.w + 1, r, c, a.view.run4 + pd.run_off, pd.nruns, dr, s1, s2);
+        sc = window_score_narrow(dot, s1, s2, pd.n, a.absolute);
+      } else {
+        long long s1, s2;
+        lane_moments<2>(a.lev, a.lev.w + 1, r, c, a.view.run4 + pd.run_off, pd.nruns, dr, s1, s2);
+        sc = window_score(dot, s1, s2, pd.n, a.absolute);
+      }
       if (better(sc, k * 25 + lane, best, border)) {
         best = sc;
         border = k * 25 + lane;
@@ -2786,10 +2845,11 @@ cudaError_t launch_pyramid(const LevelImage& src, LevelImage dst, int32_t* error
   return cudaGetLastError();
 }
 
-cudaError_t launch_prefix(const LevelImage& lev, cudaStream_t s) {
-  const int warps = lev.h, threads = 256;
-  const int blocks = (warps * 32 + threads - 1) / threads;
-  prefix_kernel<<<blocks, threads, 0, s>>>(lev);
+cudaError_t launch_prefix(const PrefixArgs& a, cudaStream_t s) {
+  int warps = 0;
+  for (int l = 0; l < a.n; ++l) warps += a.lev[l].h;
+  const int threads = 256;
+  if (warps > 0) prefix_kernel<<<(warps * 32 + threads - 1) / threads, threads, 0, s>>>(a);
   return cudaGetLastError();
 }
 
@@ -2818,7 +2878,11 @@ cudaError_t launch_track(const TrackArgs& a, int max_candidates, cudaStream_t s,
     // lists of nine take 0.17 ms with four warps and 0.22 ms with one, a 48^2
     // template's lists of three 0.78 and 0.60 ms (57,000 candidates)
     const int warps = a.sel_max <= 4 ? 1 : a.sel_max <= 8 ? 2 : kTrackWarps;
-    track_warp_kernel<<<std::min(max_candidates, 96 / warps * sms), 32 * warps, 0, s>>>(a);
+    const int grid = std::min(max_candidates, 96 / warps * sms);
+    if (a.narrow)
+      track_warp_kernel<true><<<grid, 32 * warps, 0, s>>>(a);
+    else
+      track_warp_kernel<false><<<grid, 32 * warps, 0, s>>>(a);
     return cudaGetLastError();
   }
   TrackArgs b = a;

@@ -115,9 +115,11 @@ struct TrackArgs {
   int in_slot;              // state->count index holding the input count
   double crop_row, crop_col, step, offset;
   int exact32;              // lattice arithmetic is exact in FP32 (host-checked)
+  float crop_row32, crop_col32, step32, offset32, inv_step32;  // the same in FP32
   int absolute;
   int sel_max;              // longest list of selected patches (at most 64)
   int win_rows, win_pitch;  // staged window: rows, floats per row (0: set by the launcher when it does not fit)
+  int narrow;               // the moments of every window fit the short sums of lane_moments_narrow
   int warp_lists;           // 1: the tensor cores scored all but at most two patches of every list
   // sum w S of the rotated patches of tensor-core groups (nullable),
   // kTcScoreStride per candidate, and their groups (for weff_k); the other
@@ -416,7 +418,12 @@ struct RefineArgs {
 cudaError_t launch_pyramid0(const void* src, int type, int64_t pitch_elems, int crop_row, int crop_col, LevelImage dst,
                             int32_t* error_flag, cudaStream_t s, uint32_t* quads = nullptr, int quad_tiles = 0);
 cudaError_t launch_pyramid(const LevelImage& src, LevelImage dst, int32_t* error_flag, cudaStream_t s);
-cudaError_t launch_prefix(const LevelImage& lev, cudaStream_t s);
+// Row prefixes of several levels in one launch.
+struct PrefixArgs {
+  LevelImage lev[kMaxLevels];
+  int n;
+};
+cudaError_t launch_prefix(const PrefixArgs& a, cudaStream_t s);
 cudaError_t launch_coarse(const CoarseArgs& a, int max_bh, int max_bw, cudaStream_t s, size_t smem_limit);
 cudaError_t launch_nms(const NmsArgs& a, cudaStream_t s);
 cudaError_t launch_track(const TrackArgs& a, int max_candidates, cudaStream_t s, size_t smem_limit, int sms);
