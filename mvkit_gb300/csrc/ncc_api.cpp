@@ -1548,6 +1548,12 @@ FindOutput run_find(mvg_ncc_model_s& m, const void* pixels, int type, int64_t W,
     check(launch_prefix(prefix, s), "prefix");
   }
 
+  // smallest float whose double value is >= 0.4*MinScore (the reference's
+  // FP64 comparison, matcher.cpp:582)
+  float nms_threshold = float(opt.min_score * .4);
+  if (double(nms_threshold) < opt.min_score * .4)
+    nms_threshold = std::nextafter(nms_threshold, std::numeric_limits<float>::infinity());
+
   // coarse scan + NMS
   const double scale = std::ldexp(1., int(top)), phase = (scale - 1) * .5;
   const int nplist = int(plan[top].plist.size());
@@ -1624,6 +1630,7 @@ FindOutput run_find(mvg_ncc_model_s& m, const void* pixels, int type, int64_t W,
     cs.group_of_src = d_co_gsrc;
     cs.planes = ws.planes.p;
     cs.absolute = hm.params.ignore_polarity;
+    cs.threshold = nms_threshold;
     cs.dom = dv;
     cs.crop_row = double(crop_row);
     cs.crop_col = double(crop_col);
@@ -1670,14 +1677,7 @@ FindOutput run_find(mvg_ncc_model_s& m, const void* pixels, int type, int64_t W,
     na.crop_col = double(crop_col);
     na.scale = scale;
     na.phase = phase;
-    {
-      // smallest float whose double value is >= 0.4*MinScore (the
-      // reference's FP64 comparison, matcher.cpp:582)
-      const double thr = opt.min_score * .4;
-      float f = float(thr);
-      if (double(f) < thr) f = std::nextafter(f, std::numeric_limits<float>::infinity());
-      na.threshold = f;
-    }
+    na.threshold = nms_threshold;
     na.out = ws.cand_a.p;
     na.state = st;
     na.max_candidates = cap;

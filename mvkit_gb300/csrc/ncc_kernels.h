@@ -83,6 +83,7 @@ struct CoarseTcArgs {
   const int32_t* group_of_src;
   float* planes;
   int absolute;
+  float threshold;          // scores below it are not read (nms_kernel's threshold)
   DomainView dom;
   double crop_row, crop_col, scale, phase;
 };
