@@ -2185,7 +2185,10 @@ struct MultiRefiner {
       while (j < n && order[j].owner == order[i].owner) ++j;
       const Prepared& P = *preps[size_t(order[i].owner)];
       RefineArgs ra = P.ra;
-      if (!P.owned && ws.quads_level != P.finest) ra.img.bits = 0;  // another model's level
+      if (!P.owned) {
+        if (ws.quads_level != P.finest) ra.img.bits = 0;  // another model's level
+        ra.img.quads = ws.quads.p;  // a later model may have grown the buffer
+      }
       ra.sorted = d_cand.p + i;
       ra.refined = d_ref.p + i;
       ra.refined_flag = d_flag.p + i;

@@ -38,3 +38,30 @@ def test_scores_and_poses(maxval, lowest, h, w):
     assert a.shape == b.shape
     d = np.abs(a - b)
     assert d[:, :2].max() <= 0.05 and d[:, 2].max() <= math.radians(0.05) and d[:, 3].max() <= 1e-4
+
+
+def test_models_of_different_finest_levels():
+    """One image, models whose finest levels differ: the cells' buffer of a
+    fresh thread grows with the second model, and the first one's refinement
+    reads it after the third has filled it again.  Per-model quotas: each
+    model's matches are those of its own search."""
+    import threading
+
+    import mvkit_gb300 as mg
+
+    wl = W.make_multi_workload(77, 300, 420, (56, 64, 48), (1, 1, 1), angle_range=(-A, A))
+    models = [mg.create_ncc_model(t, 3, -A, 2 * A, "auto", "use_polarity") for t in wl.templates]
+    low = [2, 1, 2]
+    out = {}
+
+    def run():
+        out["all"] = mg.find_ncc_models(wl.image, models, [-A] * 3, [2 * A] * 3, [0.6] * 3, [1] * 3, [0.5] * 3,
+                                        ["true"] * 3, [v for k in low for v in (3, k)])
+
+    t = threading.Thread(target=run)
+    t.start()
+    t.join()
+    got = np.stack(out["all"][:4], 1)
+    for k, m in enumerate(models):
+        alone = np.stack(mg.find_ncc_model(wl.image, m, -A, 2 * A, 0.6, 1, 0.5, "true", [3, low[k]]), 1)
+        assert np.array_equal(got[out["all"][4] == k], alone)
