@@ -444,7 +444,7 @@ def run_config(args) -> None:
     ach = 2.0 * d["work"] / (d["ms"] / 1e3) / 1e12 if d["ms"] else None
     roof = {"bound": "tensor", "achieved": ach, "peak": pk["tflops_sustained"], "unit": "TFLOP/s",
             "frac": ach / pk["tflops_sustained"] if ach else None, "traffic": None,
-            "kernel": "tc_track_kernel" if on_tc else "track_kernel",
+            "kernel": "tc_track_kernel" if on_tc else "track_block_kernel",
             "ms_per_launch": d["ms"] / max(1, d["launches"]),
             "cuda_core_tracking": {"achieved": 2.0 * cc["work"] / (cc["ms"] / 1e3) / 1e12 if cc["ms"] else None,
                                    "algorithmic_macs": cc["work"], "ms": cc["ms"]},
@@ -939,8 +939,8 @@ def main():
     stages = {k: v for k, v in prof.items() if isinstance(v, dict)}
     pk = peaks()
     launches_total = sum(v["launches"] for v in stages.values())
-    kernel_names = {"track": "track_kernel", "track_tc": "tc_track_kernel", "coarse": "coarse_kernel",
-                    "score": "score_kernel", "refine": "refine_kernel", "sort": "sort_kernel",
+    kernel_names = {"track": "track_block_kernel", "track_tc": "tc_track_kernel", "coarse": "coarse_kernel",
+                    "score": "score_kernel", "refine": "refine_kernel", "sort": "sort_merge_kernel",
                     "select": "select_kernel"}
     # roofline of the correlation kernel of the chosen path: tensor-core
     # tracking (its event time also covers three small grouping launches) or

@@ -7,7 +7,7 @@
 // The template dot product sum(w * (S - S_first)) runs in FP32 on the CUDA
 // cores.  The full-resolution score and the Gauss-Newton moments accumulate
 // in FP32 per thread and combine as FP32 (hi, lo) two-sum pairs; the 3x3
-// normal equations are solved in FP64 on one thread.
+// normal equations are solved in FP64, an entry per lane.
 //
 // sm_103 issues FP64 at a small fraction of the FP32 rate, so FP64 appears
 // only where the reference's decisions need it: pose lattice arithmetic (or

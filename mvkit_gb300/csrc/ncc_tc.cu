@@ -33,7 +33,7 @@
 // four window-producer warps (two slab buffers), a weight-producer
 // thread, an MMA-issue thread and four epilogue warps that also set up the
 // tiles, with two tiles in flight; accumulation is FP32 in tensor memory.  The epilogue
-// writes sum w (S - S0) per placement; track_kernel adds the exact integer
+// writes sum w S per placement; the tracking kernels add the exact integer
 // window moments and applies the reference's selection rule.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
