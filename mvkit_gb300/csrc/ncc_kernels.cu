@@ -1484,8 +1484,10 @@ __device__ __forceinline__ void inside_sums(const ImageView& img, const Original
     RawCell<Bits> raw[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int s = s0 + u * stride;
-      p[u] = s < orig.n ? __ldg(orig.dcw + s) : make_float4(0.f, 0.f, 0.f, 0.f);
+      // past the end the last sample again, not the model origin: only the
+      // samples' box was tested, and the origin of a masked template may lie
+      // outside it on a coarser level
+      p[u] = __ldg(orig.dcw + min(s0 + u * stride, orig.n - 1));
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
