@@ -1470,41 +1470,48 @@ __device__ __forceinline__ float pair_score(F2 sum, F2 sq, F2 dot, int n, int ab
 // Sums of the samples of a pose whose cells all lie inside: sum q, sum q^2,
 // sum w q.  Six samples per step, all loads issued before the arithmetic
 // (four 0.164 and 0.336 ms at 2048^2 and over a full circle, six 0.162 and
-// 0.324, eight with fewer blocks 0.163 and 0.367); each thread still adds its
-// samples in order first, first + stride, ...
+// 0.324, eight with fewer blocks 0.163 and 0.367); each thread adds its samples
+// in order first, first + stride, ...  The samples past the last whole step go
+// one by one: only cells of real samples may be loaded, since the samples' box
+// is what was tested and the model origin of a masked template may lie outside
+// it on a coarser level.
 constexpr int kScoreUnroll = 6;
 constexpr int kTeamUnroll = 8;  // passes of a cluster: more registers per thread
+template <int Bits> struct InsideSample {
+  float w, fy, fx;
+  RawCell<Bits> raw;
+  __device__ __forceinline__ void load(const ImageView& img, const LocalPose& L, const float4& p) {
+    const float y = __fadd_rn(L.fr, fms2(L.ca, p.x, L.sa, p.y));
+    const float x = __fadd_rn(L.fc, fma2(L.ca, p.y, L.sa, p.x));
+    const int iy = split_floor(y, fy), ix = split_floor(x, fx);
+    w = p.z;
+    raw.load(img, L.C0 + ix, L.R0 + iy);
+  }
+  __device__ __forceinline__ void add(float offset, float (&acc)[4]) const {
+    const float q = __fsub_rn(cell_value(raw.cell(), fy, fx), offset);
+    acc[0] += q;
+    acc[1] = fmaf(q, q, acc[1]);
+    acc[2] = fmaf(w, q, acc[2]);
+  }
+};
 template <int Bits, int Unroll>
 __device__ __forceinline__ void inside_sums(const ImageView& img, const OriginalView& orig, const LocalPose& L,
                                             float offset, int first, int stride, float (&acc)[4]) {
-  constexpr int U = Unroll;
-  for (int s0 = first; s0 < orig.n; s0 += U * stride) {
-    float4 p[U];
-    float fy[U], fx[U];
-    RawCell<Bits> raw[U];
+  int s = first;
+  for (; s + (Unroll - 1) * stride < orig.n; s += Unroll * stride) {
+    float4 p[Unroll];
+    InsideSample<Bits> at[Unroll];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      // past the end the last sample again, not the model origin: only the
-      // samples' box was tested, and the origin of a masked template may lie
-      // outside it on a coarser level
-      p[u] = __ldg(orig.dcw + min(s0 + u * stride, orig.n - 1));
-    }
+    for (int u = 0; u < Unroll; ++u) p[u] = __ldg(orig.dcw + s + u * stride);
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const float y = __fadd_rn(L.fr, fms2(L.ca, p[u].x, L.sa, p[u].y));
-      const float x = __fadd_rn(L.fc, fma2(L.ca, p[u].y, L.sa, p[u].x));
-      const int iy = split_floor(y, fy[u]), ix = split_floor(x, fx[u]);
-      raw[u].load(img, L.C0 + ix, L.R0 + iy);
-    }
+    for (int u = 0; u < Unroll; ++u) at[u].load(img, L, p[u]);
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      if (s0 + u * stride >= orig.n) break;
-      const Cell v = raw[u].cell();
-      const float q = __fsub_rn(cell_value(v, fy[u], fx[u]), offset);
-      acc[0] += q;
-      acc[1] = fmaf(q, q, acc[1]);
-      acc[2] = fmaf(p[u].z, q, acc[2]);
-    }
+    for (int u = 0; u < Unroll; ++u) at[u].add(offset, acc);
+  }
+  for (; s < orig.n; s += stride) {
+    InsideSample<Bits> at;
+    at.load(img, L, __ldg(orig.dcw + s));
+    at.add(offset, acc);
   }
 }
 
