@@ -1842,6 +1842,11 @@ FindOutput run_find(mvg_ncc_model_s& m, const void* pixels, int type, int64_t W,
   geom.top = -base.orow - .5;
   geom.bottom = double(base.height) - base.orow - .5;
   geom.area = double(base.width) * double(base.height);
+  if (std::max(std::abs(opt.angle_start), std::abs(opt.angle_start + opt.angle_extent)) > 12.6) {
+    // more than two turns from zero: angles relative to the start's direction
+    geom.angle_from = opt.angle_start;
+    geom.angle_to = std::atan2(std::sin(opt.angle_start), std::cos(opt.angle_start));
+  }
   const double fscale = std::ldexp(1., int(finest)), fphase = (fscale - 1) * .5;
   ImageView fine{lev[finest].v, lw[finest], lh[finest]};
   if (quad.bits) {

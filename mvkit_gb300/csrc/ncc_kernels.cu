@@ -2073,37 +2073,19 @@ __global__ void __launch_bounds__(256) sort_merge_kernel(SortArgs a, int seg, co
 }
 
 // ----------------------------------------------------------------- overlap
-// FP32 cos and sin of an FP64 angle, each within an ulp or two of the FP64
-// value at any angle: whole turns are taken off in FP64 (2 pi in two parts,
-// Cody and Waite) and what the FP32 angle drops of the rest goes in to first
-// order.  Angles beyond 2^30 take FP64 sincos, out of line.
-__device__ __noinline__ float2 sincos_far(double angle) {
-  double s, c;
-  sincos(angle, &s, &c);
-  return make_float2(float(s), float(c));
-}
-__device__ __forceinline__ void sincos_any(double angle, float& s, float& c) {
-  if (!(fabs(angle) < 1073741824.)) {
-    const float2 far = sincos_far(angle);
-    s = far.x;
-    c = far.y;
-    return;
-  }
-  const double turns = rint(dmul(angle, 0.15915494309189535));
-  const double rest = __fma_rn(-turns, 2.4492935982947064e-16, __fma_rn(-turns, 6.283185307179586, angle));
-  const float hi = float(rest), lo = float(dsub(rest, double(hi)));
-  float sh, ch;
-  sincosf(hi, &sh, &ch);
-  s = __fmaf_rn(ch, lo, sh);
-  c = __fmaf_rn(-sh, lo, ch);
-}
-
 // Rotated rectangle of a pose: FP32 cos/sin and a conservative FP32 box for
-// the cheap disjointness test.  FP64 sincos is left to the exact overlap,
-// which few pairs need: one per sorted candidate took 18 us of a small find.
+// the cheap disjointness test.  The angle is brought near zero in FP64 (the
+// search range may lie anywhere) and what its float drops goes in to first
+// order, so cos and sin are within an ulp or two of the FP64 ones.  FP64 sincos
+// is left to the exact overlap, which few pairs need.
 __device__ RectAux make_rect(const Cand& m, const RectGeom& g) {
   RectAux r;
-  sincos_any(m.angle, r.sa, r.ca);
+  const double angle = dadd(dsub(m.angle, g.angle_from), g.angle_to);
+  const float hi = float(angle), lo = float(dsub(angle, double(hi)));
+  float sh, ch;
+  sincosf(hi, &sh, &ch);
+  r.sa = __fmaf_rn(ch, lo, sh);
+  r.ca = __fmaf_rn(-sh, lo, ch);
   float x0 = INFINITY, y0 = INFINITY, x1 = -INFINITY, y1 = -INFINITY;
   const double xs[2] = {g.left, g.right}, ys[2] = {g.top, g.bottom};
   for (double x : xs)

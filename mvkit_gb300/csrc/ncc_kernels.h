@@ -356,6 +356,9 @@ struct Refine4Args {
 // (src/ncc_matching/matcher.cpp:257-258).
 struct RectGeom {
   double left, right, top, bottom, area;
+  // angle - angle_from + angle_to is the same direction and small (both zero
+  // for ordinary ranges)
+  double angle_from = 0, angle_to = 0;
 };
 
 // Candidate sort (score descending, then row, column, angle).  keys / idx:
