@@ -1831,8 +1831,8 @@ __device__ __noinline__ double sim_score(const Refine4Args& a, SimLocal& loc, co
 // the reference's refinement_step), an FP64 Gauss-Jordan solve with partial
 // pivoting (a matrix entry per lane of warp 0), the step clipped to the
 // limits, and up to four halvings; a step is taken only when the score
-// strictly increases.  64 poses of a 161^2 template: 2.29 -> 1.52 ms
-// (3000x4096 image; 1.80 with one block per pose).
+// strictly increases.  Bound by the latency of the passes.  64 poses of a
+// 161^2 template in a 3000x4096 image: 2.17 -> 1.56 ms (1.79 with one block per pose).
 constexpr int kRefine4Threads = 256;  // of a team of C blocks
 
 template <class T, int C>
@@ -2967,9 +2967,17 @@ cudaError_t launch_adjoint(const AdjointArgs& a, cudaStream_t s) {
 
 cudaError_t launch_refine4(const Refine4Args& a, cudaStream_t s, int sms) {
   if (a.n <= 0) return cudaSuccess;
-  // few poses: four SMs share the samples of one; from about a pose per SM on
-  // the GPU is full and the cluster barriers only cost
-  const bool team = a.n < sms;
+  // Four SMs share the samples of a pose where rows a multiple of 256 bytes
+  // apart fall on few L1 sets, so that a rotated pose's gathers on one SM push
+  // one another out: 32 poses at all angles, one block -> cluster, rows 2560
+  // apart, 96^2 0.74 -> 0.80, 128^2 1.17 -> 1.04, 200^2 2.36 -> 2.00, 256^2 3.53
+  // -> 2.87 ms; 4096 apart, 128^2 1.28 -> 1.04, 256^2 4.02 -> 3.07.  Upright poses
+  // do not gain there (4096 apart, 128^2 0.92 -> 1.11, 256^2 3.20 -> 3.21), and
+  // other row lengths lose at every angle (3000 apart, 96^2 0.62 -> 0.78, 161^2
+  // 1.21 -> 1.32, 256^2 3.39 -> 3.32), as do full GPUs: from a pose per SM on the
+  // cluster barriers only cost.
+  const int64_t row_bytes = a.img.pitch * (a.img.type == 1 ? 2 : 1);
+  const bool team = a.n < sms && a.orig.n >= 12288 && row_bytes % 256 == 0;
   const int grid = team ? 4 * a.n : a.n, threads = team ? kRefine4Threads / 4 : kRefine4Threads;
   if (a.img.type == 1)
     team ? refine4_kernel<uint16_t, 4><<<grid, threads, 0, s>>>(a) : refine4_kernel<uint16_t, 1><<<grid, threads, 0, s>>>(a);
