@@ -179,8 +179,7 @@ __device__ __forceinline__ double div_small(double d, double n, double r) {
 // per lane, and handed to the chain by shuffles.  An FP64 instruction holds
 // an SM quarter's pipe for some 64 cycles however many lanes it has, so the
 // chain's five operations per sample of the mean and one for each sum bound
-// it.  384 rasters of a 128^2 template: 17.7 -> 4.6 ms (profiled; one
-// thread per raster with a division in the chain before, 9.4 without it).
+// it.  384 rasters of a 128^2 template: 17.7 -> 4.6 ms (profiled).
 __global__ void __launch_bounds__(32) raster_moments_kernel(const RasterJob* jobs, const int* samples, const int2* rc,
                                                             double* v, const double* __restrict__ reciprocals,
                                                             int* flag, float* fwsum, int4* bounds) {

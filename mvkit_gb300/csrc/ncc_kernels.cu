@@ -1,9 +1,13 @@
 // CUDA kernels of the GB300 NCC find path (sm_103a).
 //
 // Numerics.  Every pyramid value is an integer sum of 4^k input pixels, held
-// exactly in float.  Window moments (sum S, sum S^2) come from int64 row
-// prefix sums, so the variance numerator n*sum(S^2) - (sum S)^2 is exact and
-// the "variance <= 0 -> no score" rule of the reference is decided exactly.
+// exactly in float.  Window moments (sum S, sum S^2) come from row prefix sums:
+// int64, or uint32 modulo 2^32 where the host found that a run's sum S^2 stays
+// below 2^32 (its longest run times the level's largest value squared), so that
+// a difference of two entries is exact; windows whose sums and variance numerator
+// are bounded as well are summed in 32 bits (TrackArgs::narrow).  Either way the
+// variance numerator n*sum(S^2) - (sum S)^2 is exact and the "variance <= 0 ->
+// no score" rule of the reference is decided exactly.
 // The template dot product sum(w * (S - S_first)) runs in FP32 on the CUDA
 // cores.  The full-resolution score and the Gauss-Newton moments accumulate
 // in FP32 per thread and combine as FP32 (hi, lo) two-sum pairs; the 3x3
@@ -304,8 +308,7 @@ __device__ __forceinline__ void prefix_row(const float* __restrict__ row, int w,
 
 // Row prefix sums {sum S, sum S^2}, one warp per row, the rows of every level
 // of the find in one launch (the widest level first): the levels' chains of
-// row steps run side by side.  Three levels of 2048^2: 0.043 -> 0.010 ms (a launch
-// per level, 32 columns per step before).
+// row steps run side by side.  Three levels of 2048^2: 0.043 -> 0.010 ms.
 __global__ void prefix_kernel(const __grid_constant__ PrefixArgs a) {
   int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, l = 0;
   while (l < a.n && warp >= a.lev[l].h) warp -= a.lev[l++].h;
@@ -876,8 +879,7 @@ __device__ __forceinline__ float track_tc_dot(const TrackArgs& a, const PatchDes
 // correlated first, by the block.  Bound by the instructions around the
 // prefix loads and their latency.  2048^2 u8, 128^2 template, two steps: 0.27
 // -> 0.16 ms; 57,000 candidates of a 48^2 template over a full circle: 1.03 ->
-// 0.56 ms (one 256-thread block per possible candidate before, each step's
-// lanes on five image rows; 0.17 and 0.61 with 64-bit sums and indices).
+// 0.56 ms.
 
 // Dots of patch k of candidate cd, sum w (S - S0), by the whole block, to
 // out[position].  Kept out of line: few candidates need it, and its registers
@@ -988,9 +990,7 @@ __global__ void __launch_bounds__(32 * kTrackWarps, 8) track_warp_kernel(const _
 // register tiles leave (set-up and staging a quarter of them, dots and
 // moments 60 %).  uint16 lists, two steps at 2048^2 with a 128^2 template
 // (3.1 G multiply-adds): 1.98 -> 0.92 ms; three at 4096^2 with 256^2 (21 G):
-// 40 -> 5.2 ms (one shared-memory read and one weight read per multiply-add,
-// and a 256-thread block per possible candidate, before; 1.09 and 5.8 with
-// 256-thread blocks here).
+// 40 -> 5.0 ms.
 __global__ void __launch_bounds__(512) track_block_kernel(TrackArgs a) {
   extern __shared__ float smem[];
   __shared__ int s_row[kTrackMaxSel], s_col[kTrackMaxSel];
@@ -1468,13 +1468,12 @@ __device__ __forceinline__ float pair_score(F2 sum, F2 sq, F2 dot, int n, int ab
 }
 
 // Sums of the samples of a pose whose cells all lie inside: sum q, sum q^2,
-// sum w q.  Six samples per step, all loads issued before the arithmetic
-// (four 0.164 and 0.336 ms at 2048^2 and over a full circle, six 0.162 and
-// 0.324, eight with fewer blocks 0.163 and 0.367); each thread adds its samples
-// in order first, first + stride, ...  The samples past the last whole step go
-// one by one: only cells of real samples may be loaded, since the samples' box
-// is what was tested and the model origin of a masked template may lie outside
-// it on a coarser level.
+// sum w q.  Six samples per step, all loads issued before the arithmetic (full
+// circle 0.293 ms, 4096^2 uint16 1.12; four 0.309 and 1.48, eight with ten blocks
+// per SM 0.297 and 1.11); each thread adds its samples in order first, first +
+// stride, ...  The samples past the last whole step go one by one: only cells of
+// real samples may be loaded, since the samples' box is what was tested and the
+// model origin of a masked template may lie outside it on a coarser level.
 constexpr int kScoreUnroll = 6;
 constexpr int kTeamUnroll = 8;  // passes of a cluster: more registers per thread
 template <int Bits> struct InsideSample {
@@ -1560,9 +1559,8 @@ __device__ __forceinline__ double continuous_pass(const ImageView& img, const Or
 
 // Full-resolution score of every candidate.  Bound by the latency of the
 // gathers and the instructions around them (some 55 per 32 samples, one
-// gather).  Quads against row-major values: 4096^2 uint16 with a 256^2
-// template 3.17 -> 1.35 ms, 1024x1280 full circle with 48^2 0.52 -> 0.32 ms
-// (0.40 of it the folded reduction), 2048^2 uint8 0.172 -> 0.162 ms.
+// gather).  4096^2 uint16 with a 256^2 template 3.17 -> 1.12 ms, 1024x1280
+// full circle with 48^2 0.52 -> 0.29 ms, 2048^2 uint8 0.172 -> 0.163 ms.
 template <int Bits> __global__ void __launch_bounds__(128, 12) score_kernel(ScoreArgs a) {
   __shared__ BlockTotals<4> tot;
   __shared__ LocalPose lp;
@@ -2747,11 +2745,10 @@ template <int C> __device__ __noinline__ void recovery_search(const RefineArgs& 
 }
 
 // refine_candidate (src/ncc_matching/matcher.cpp:878-1061) for one queued
-// candidate per block.  Bound by the latency of a chain of passes: gathers,
-// two reductions and FP64 algebra each.  Five 128^2 candidates (six
-// Gauss-Newton passes and four scores each): 0.385 -> 0.164 ms (19 shuffle trees
-// per warp and once more on warp 0, FP64 steps on one thread, one sample at a
-// time before).
+// candidate per block, or per cluster of C blocks (launch_refine says when).
+// Bound by the latency of a chain of passes: gathers, two reductions and FP64
+// algebra each.  Five 128^2 candidates (six Gauss-Newton passes and four scores
+// each): 0.385 -> 0.143 ms.
 template <int Bits, int C>
 __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kRefineThreads / C)
     refine_kernel(const __grid_constant__ RefineArgs a) {
@@ -2918,9 +2915,10 @@ cudaError_t launch_track(const TrackArgs& a, int max_candidates, cudaStream_t s,
   // candidate costs more than the work when the budget is large (65536
   // blocks: about 60 us)
   if (a.warp_lists) {
-    // a warp for every four patches of the longest list: a 128^2 template's
-    // lists of nine take 0.17 ms with four warps and 0.22 ms with one, a 48^2
-    // template's lists of three 0.78 and 0.60 ms (57,000 candidates)
+    // a warp for every four patches of the longest list, against one and four
+    // warps for every list: 128^2 templates at 2048^2 0.158 / 0.171 / 0.169 ms,
+    // 96^2 0.129 / 0.139 / 0.138; short lists would take one warp alone (64^2
+    // 0.224 / 0.197 / 0.238, 57,000 candidates of 48^2 0.56 / 0.46 / 0.75)
     const int warps = a.sel_max <= 4 ? 1 : a.sel_max <= 8 ? 2 : kTrackWarps;
     const int grid = std::min(max_candidates, 96 / warps * sms);
     if (a.narrow)
@@ -2940,9 +2938,12 @@ cudaError_t launch_track(const TrackArgs& a, int max_candidates, cudaStream_t s,
   smem += tables;
   if (const cudaError_t e = reserve_dynamic_smem(reinterpret_cast<const void*>(track_block_kernel), smem)) return e;
   // 128 registers a thread leave an SM 16 warps: in as many blocks as the
-  // window lets in, so that their phases overlap (four blocks of 128 threads
-  // 0.92, two of 256 1.09 ms at 2048^2; one of 256 7.0, of 512 5.8 ms where
-  // the window fills the SM)
+  // window lets in, so that their phases overlap.  One block size for all sizes,
+  // 128 / 256 / 512 threads, uint16 lists at 2048^2 by the windows of their larger
+  // level: 41 KB 0.40 / 0.44 / 0.56 ms, 62 KB 0.32 / 0.32 / 0.37, 86 KB 0.69 /
+  // 0.57 / 0.67, 113 KB 0.15 / 0.09 / 0.07, 164 KB 1.05 / 0.73 / 0.64.  Lines
+  // drawn where four and two blocks still fit instead (57 and 112 KB) gave 4 % at
+  // 101 KB and took 7 % at 55 KB, where the lists were short.
   const int threads = smem > 100 * 1024 ? 512 : smem > 50 * 1024 ? 256 : 128;
   track_block_kernel<<<std::min(max_candidates, 16 * sms), threads, smem, s>>>(b);
   return cudaGetLastError();
@@ -3055,9 +3056,11 @@ template <int C> void refine_launch(const RefineArgs& a, int batch_limit, cudaSt
 }  // namespace
 
 cudaError_t launch_refine(const RefineArgs& a, int batch_limit, cudaStream_t s) {
-  // a large template's samples pay for the cluster's barriers: 128^2 0.182
-  // (one block) and 0.164 ms (cluster), 256^2 0.49 and 0.40, but 64^2 0.086
-  // and 0.097, 48^2 over a full circle 0.106 and 0.122
+  // a large template's samples pay for the cluster's barriers.  One block ->
+  // cluster, four candidates of a uint8 search: 64^2 0.080 -> 0.090 ms, 96^2
+  // 0.088 -> 0.096, 104^2 0.092 -> 0.098, 112^2 0.127 -> 0.131, 128^2 0.123 ->
+  // 0.115, 160^2 0.186 -> 0.164, 256^2 0.36 -> 0.28; of a uint16 one: 104^2 0.111
+  // -> 0.109, 112^2 0.129 -> 0.121.  Long candidate lists cross over near 88^2.
   if (a.orig.n >= 12288)
     refine_launch<4>(a, batch_limit, s);
   else

@@ -755,7 +755,7 @@ __global__ void tc_planes_kernel(LevelImage lev, __half* planes, int pitch, floa
 // (x 64 likewise), which the centring columns of the window multiply.  The
 // halves are multiples of 2^-24, so the sums are added as integers: any order
 // gives the same.  A 128^2 template's three plans (270 patches of 90 groups
-// at the finest): 76 -> 1.5 ms with the host's work around it (on the host before).
+// at the finest): 76 -> 1.5 ms with the host's work around it.
 __global__ void __launch_bounds__(256) tc_weights_kernel(const TcWeightJob* jobs, const int2* __restrict__ sw,
                                                          unsigned long long* rows, TcWeightSums* sums) {
   const TcWeightJob J = jobs[blockIdx.x];
